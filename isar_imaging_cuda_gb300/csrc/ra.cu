@@ -26,6 +26,7 @@
 
 #include <type_traits>
 
+#include "cells_fixed.h"
 #include "fft.cuh"
 #include "isar_kernels.h"
 
@@ -193,11 +194,19 @@ __global__ void k_zero_shift(double* __restrict__ S, int64_t* __restrict__ SQ, i
 
 // S[row] += sh and SQ[row] = S[row] / N as a 64-bit fixed-point fraction,
 // once per row (one thread), so that the row transforms read SQ directly.
-__device__ __forceinline__ void add_shift(double* S, int64_t* SQ, size_t row, float sh, int N)
+template <int N>
+__device__ __forceinline__ void add_shift(double* S, int64_t* SQ, size_t row, float sh)
 {
     const double v = S[row] + (double)sh;
     S[row] = v;
-    SQ[row] = frac_to_fixed(v / (double)N);
+    SQ[row] = cells_to_fixed((uint64_t)__double_as_longlong(v), ilog2c(N));
+}
+
+// The slope SQ of one shift sh.
+template <int N>
+__device__ __forceinline__ int64_t shift_slope(float sh)
+{
+    return cells_to_fixed((uint64_t)__double_as_longlong((double)sh), ilog2c(N));
 }
 
 // Standalone HPC (stage test entry): x *= exp(j*2*pi*alpha_m*n^2).
@@ -266,27 +275,32 @@ __device__ __forceinline__ void pair_add(float& h, float& l, float h2, float l2)
     h = t;
 }
 
-// Block total of compensated float pairs as a double; valid in thread 0.
-// Float arithmetic throughout (FP64 issues slowly on this part) with the
-// precision of a double sum.
+// Block totals of three compensated float pairs as floats, valid in threads
+// 0, 1 and 2 (total j in thread j); one barrier.  Float arithmetic throughout
+// with the precision of a double sum (FP64 issues slowly on this part: only
+// the final rounding of the three totals uses it, in one warp).
 template <int T>
-__device__ __forceinline__ double block_sum_pair0(float h, float l, float2* red)
+__device__ __forceinline__ float block_sum_pair3(float* h, float* l, float2 (*red)[32])
 {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        pair_add(h, l, __shfl_xor_sync(0xffffffffu, h, o), __shfl_xor_sync(0xffffffffu, l, o));
-    double r = (double)h + (double)l;
+    for (int j = 0; j < 3; ++j) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            pair_add(h[j], l[j], __shfl_xor_sync(0xffffffffu, h[j], o), __shfl_xor_sync(0xffffffffu, l[j], o));
+    }
     constexpr int W = T / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if constexpr (W > 1) {
-        const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-        if (lane == 0) red[w] = make_float2(h, l);
+        if (lane < 3) red[lane][w] = make_float2(lane == 0 ? h[0] : lane == 1 ? h[1] : h[2],
+                                                 lane == 0 ? l[0] : lane == 1 ? l[1] : l[2]);
         __syncthreads();
-        if (threadIdx.x == 0) {
-            float H = red[0].x, L = red[0].y;
-            for (int i = 1; i < W; ++i) pair_add(H, L, red[i].x, red[i].y);
-            r = (double)H + (double)L;
-        }
-        __syncthreads();
+    }
+    float r = 0.0f;
+    if (w == 0 && lane < 3) {
+        float H = lane == 0 ? h[0] : lane == 1 ? h[1] : h[2], L = lane == 0 ? l[0] : lane == 1 ? l[1] : l[2];
+#pragma unroll 1
+        for (int i = 1; i < W; ++i) pair_add(H, L, red[lane][i].x, red[lane][i].y);
+        r = (float)((double)H + (double)L);
     }
     return r;
 }
@@ -303,25 +317,31 @@ __device__ __forceinline__ float csum3(float hi, float lo, float x)
     return t + e;
 }
 
+// A pair's shift in cells and its fixed-point phase slope.
+struct RaShift {
+    float sh;
+    int64_t slope;
+};
+
 // Correlates the RMS envelopes a = sqrt(ea), b = sqrt(eb) as the reference
 // does, C2R(R2C(a) .* conj(R2C(b))) -> ifftshift -> argmax|.| -> parabolic
-// fix (range_alignment.cu:50-66, :121-168), and returns the shift (all
-// threads).  The FFT locates the peak; the three samples of the parabola are
+// fix (range_alignment.cu:50-66, :121-168), stores the shift to *shift_out
+// (given: reads it from there instead) and returns it in all threads.  One
+// call per kernel.  The FFT locates the peak; the three samples of the parabola are
 // then evaluated directly, sum_n a[n] b[n - tau] with error-free float
 // accumulation, because the second difference of a broad correlation peak
 // magnifies FFT rounding into ~1e-4-cell shift errors.  A(n), B(n) return
 // the amplitudes a[n], b[n] (shared-memory reads, n in [0, N)); sm_f is the
 // FFT scratch.
 template <int N, class AmpA, class AmpB, class Tw>
-__device__ float ra_correlate_f(AmpA A, AmpB B, float* sm_f, int lt, const Tw& tw)
+__device__ RaShift ra_correlate_f(AmpA A, AmpB B, float* sm_f, int lt, const Tw& tw, float* shift_out, int given)
 {
     using F = FFTShape<N>;
     constexpr int T = F::T;
     float2* sm = reinterpret_cast<float2*>(sm_f);
     __shared__ ArgKey red[32];
-    __shared__ float2 redp[32];
-    __shared__ float s_res;
-    __shared__ int s_pos;
+    __shared__ float2 redp[3][32];
+    __shared__ RaShift s_res;
     // z = a + i b, forward FFT, spectrum kept in the scratch (padded slots)
     team_fft<N, false>([&](int i) { return make_float2(A(i), B(i)); },
                        [&](int i, float2 v, int) { sm[fpad(i)] = v; }, sm, lt, tw);
@@ -348,10 +368,7 @@ __device__ float ra_correlate_f(AmpA A, AmpB B, float* sm_f, int lt, const Tw& t
         row_fft<N, true, true>(csrc, cdst, sm, lt, tw, NoHook{});   // output order is irrelevant to an argmax
     else
         team_fft<N, true>(csrc, cdst, sm, lt, tw);
-    best = block_argmax<T>(best, red);
-    if (lt == 0) s_pos = best.i;
-    __syncthreads();
-    const int pos = s_pos;
+    const int pos = block_argmax<T>(best, red).i;
     const int tau = (pos + N / 2) & (N - 1);
     // f_j = sum_n a[n] b[n - (tau + j)], j = -1, 0, 1
     float h[3] = {0.0f, 0.0f, 0.0f}, l[3] = {0.0f, 0.0f, 0.0f};
@@ -362,33 +379,37 @@ __device__ float ra_correlate_f(AmpA A, AmpB B, float* sm_f, int lt, const Tw& t
 #pragma unroll
         for (int j = 0; j < 3; ++j) acc_prod(a, B((n - tau - (j - 1)) & (N - 1)), h[j], l[j]);
     }
-    double f[3];
-#pragma unroll
-    for (int j = 0; j < 3; ++j) f[j] = block_sum_pair0<T>(h[j], l[j], redp);
-    if (lt == 0) {
+    const float f = block_sum_pair3<T>(h, l, redp);
+    if (lt < 32) {
         // the reference keeps the correlation in a float buffer and fits the
         // parabola in float (binomialFixDevice, range_alignment.cu:121-131)
-        const float f1 = (float)f[0], f2 = (float)f[1], f3 = (float)f[2];
+        const float f1 = __shfl_sync(0xffffffffu, f, 0), f2 = __shfl_sync(0xffffffffu, f, 1),
+                    f3 = __shfl_sync(0xffffffffu, f, 2);
         const float fa = __fdiv_rn(__fsub_rn(__fadd_rn(f1, f3), __fmul_rn(2.0f, f2)), 2.0f);
         const float fb = __fdiv_rn(__fsub_rn(f3, f1), 2.0f);
         const float delta = __fdiv_rn(-fb, __fmul_rn(2.0f, fa));
-        s_res = __fsub_rn(__fadd_rn((float)pos, delta), (float)N / 2);
+        float sh = __fsub_rn(__fadd_rn((float)pos, delta), (float)N / 2);
+        if (given) sh = *shift_out;   // injected by the caller (test hook)
+        if (lt == 0) {
+            if (!given) *shift_out = sh;
+            s_res.sh = sh;
+            s_res.slope = shift_slope<N>(sh);
+        }
     }
     __syncthreads();
-    const float r = s_res;
-    __syncthreads();
-    return r;
+    return s_res;
 }
 
 // ra_correlate_f on squared envelopes: ea, eb are adjacent N-float shared
 // arrays, replaced in place by the amplitudes a = sqrt(ea), b = sqrt(eb).
 template <int N, class Tw>
-__device__ float ra_correlate(float* ea, float* sm_f, int lt, const Tw& tw)
+__device__ RaShift ra_correlate(float* ea, float* sm_f, int lt, const Tw& tw, float* shift_out, int given)
 {
     float* eb = ea + N;
     for (int i = lt; i < 2 * N; i += FFTShape<N>::T) ea[i] = sqrtf(ea[i]);
     __syncthreads();
-    return ra_correlate_f<N>([&](int n) { return ea[n]; }, [&](int n) { return eb[n]; }, sm_f, lt, tw);
+    return ra_correlate_f<N>([&](int n) { return ea[n]; }, [&](int n) { return eb[n]; }, sm_f, lt, tw, shift_out,
+                             given);
 }
 
 // s + x accumulated error-free into (s, c) (TwoSum).
@@ -521,10 +542,8 @@ k_ra_pair(const float2* __restrict__ x, float2* xw, const float* __restrict__ wi
     if (left_next)
         for (int i = lt; i < N; i += F::T) left_next[(size_t)j * N + i] = ea[i];
     __syncthreads();
-    const float shc = ra_correlate<N>(ea, sm_f, lt, tws);
-    const float sh = given ? shift_out[j] : shc;   // given: shifts injected by the caller (test hook)
-    if (lt == 0 && !given) shift_out[j] = sh;
-    for (int m = lt; m < s; m += F::T) add_shift(S, SQ, (size_t)(2 * j + 1) * s + m, sh, N);
+    const float sh = ra_correlate<N>(ea, sm_f, lt, tws, shift_out + j, given).sh;
+    for (int m = lt; m < s; m += F::T) add_shift<N>(S, SQ, (size_t)(2 * j + 1) * s + m, sh);
 }
 
 // Level >= 1, many rows per group: CTA b transforms rpc rows of R_k
@@ -610,10 +629,8 @@ k_ra_corr(const float* __restrict__ E, double* __restrict__ S, int64_t* __restri
     RaTw<N>::fill(twt, tw, lt, F::T);
     for (int i = lt; i < 2 * N; i += F::T) ea[i] = E[(size_t)2 * j * N + i];
     __syncthreads();
-    const float shc = ra_correlate<N>(ea, sm_f, lt, RaTw<N>{twt});
-    const float sh = given ? shift_out[j] : shc;
-    if (lt == 0 && !given) shift_out[j] = sh;
-    for (int m = lt; m < s; m += F::T) add_shift(S, SQ, (size_t)(2 * j + 1) * s + m, sh, N);
+    const float sh = ra_correlate<N>(ea, sm_f, lt, RaTw<N>{twt}, shift_out + j, given).sh;
+    for (int m = lt; m < s; m += F::T) add_shift<N>(S, SQ, (size_t)(2 * j + 1) * s + m, sh);
 }
 
 // ---------------------------------------------------------------------------
@@ -731,13 +748,9 @@ k_ra_spec0(const float2* x, float2* xw, const float* __restrict__ win, const int
             sm, lt, tws, NoHook{});
     }
     __syncthreads();
-    const float shc = ra_correlate_f<N>([&](int n) { return ca[pc(n)].x; }, [&](int n) { return cb[pc(n)].x; },
-                                        reinterpret_cast<float*>(sm), lt, tws);
-    const float sh = given ? shift_out[j] : shc;   // given: shifts injected by the caller (test hook)
-    if (lt == 0) {
-        if (!given) shift_out[j] = sh;
-        add_shift(S, SQ, (size_t)2 * j + 1, sh, N);
-    }
+    const auto [sh, slope] = ra_correlate_f<N>([&](int n) { return ca[pc(n)].x; }, [&](int n) { return cb[pc(n)].x; },
+                                               reinterpret_cast<float*>(sm), lt, tws, shift_out + j, given);
+    if (lt == 0) add_shift<N>(S, SQ, (size_t)2 * j + 1, sh);
     if (wout == nullptr) return;
     // Z = FFT(w_even + j w_odd) in place (both transforms read all their
     // inputs before their first barrier and write their outputs after the
@@ -755,7 +768,7 @@ k_ra_spec0(const float2* x, float2* xw, const float* __restrict__ win, const int
     __syncthreads();
     LinPhase<N> h, r;
     h.init(kHalfCellDown<N>, lt);
-    r.init(frac_to_fixed((double)sh / (double)N), lt);
+    r.init(slope, lt);
     float2* w = wout + (size_t)j * N;
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
@@ -810,13 +823,12 @@ k_ra_spec(const float2* __restrict__ wprev, float2* __restrict__ wout, double* _
         },
         sm, lt, tws);
     __syncthreads();
-    const float shc = ra_correlate_f<N>([&](int n) { return ea[n]; }, [&](int n) { return eb[n]; }, sm_f, lt, tws);
-    const float sh = given ? shift_out[j] : shc;
-    if (lt == 0 && !given) shift_out[j] = sh;
-    for (int m = lt; m < s; m += F::T) add_shift(S, SQ, (size_t)(2 * j + 1) * s + m, sh, N);
+    const auto [sh, slope] = ra_correlate_f<N>([&](int n) { return ea[n]; }, [&](int n) { return eb[n]; }, sm_f, lt,
+                                               tws, shift_out + j, given);
+    for (int m = lt; m < s; m += F::T) add_shift<N>(S, SQ, (size_t)(2 * j + 1) * s + m, sh);
     if (wout == nullptr) return;
     LinPhase<N> r;
-    r.init(frac_to_fixed((double)sh / (double)N), lt);
+    r.init(slope, lt);
     float2* w = wout + (size_t)j * N;
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
