@@ -437,34 +437,64 @@ k_af_persist(const float2* __restrict__ cut, const int* __restrict__ bins, const
 
 // ---------------------------------------------------------------------------
 // Cluster-resident autofocus: the same iteration as k_af_persist, with all
-// state of one frame held in the shared memory of one thread-block cluster.
+// state of one frame held in the shared memory of one thread-block cluster
+// and every transform inside one warp.
 //
-// CTA r of a cluster of CL owns bins [r*bpc, r*bpc + nb), bpc = ceil(U/CL),
-// processed TEAMS at a time (one team of M/16 threads per bin).  Two chunk
-// slots of TEAMS columns are cached in shared memory; a CTA owning more
-// chunks reloads the ones past the first slot from the cut every iteration.
-// Per iteration: each CTA accumulates P[m] = sum over its bins of
-// conj(g) .* IFFT(T .* |T|)/M, T = FFT(phase .* g); cluster barrier; CTA r
-// reduces rows [r*M/CL, (r+1)*M/CL) over the CL partials (distributed shared
-// memory, fixed rank order), normalises and stores the new phase into every
-// CTA's copy; cluster barrier.  The entropy of the selected bins,
-// E = ln S1 - ln 2 * S2/S1 with S1 = sum |T|^2, S2 = sum |T|^2 log2 |T|^2, comes out of
-// the same epilogue and drives the optional stop criterion.
-// Only hardware cluster barriers: no spin-waits.
+// CTA r of a cluster of CL owns bins [r*bpc, r*bpc + nb), bpc = ceil(U/CL).
+// L lanes own one bin (a warp; half a warp at 128 pulses): element
+// m = l + L i lives in lane l, register i (i < P, M = P L).  The forward
+// transform runs as
+//   DFT_P over i -> k1, twiddle W_M^(l k1), exchange through the warp's tile:
+//   lane (k1, q) gets l = q + Q b (Q = L / P), DFT_P over b -> c, twiddle
+//   W_L^(q c), DFT_Q over q between neighbouring lanes by shuffles (AfCross),
+// and the inverse is its mirror image from that order back to pulse order, so
+// T |T| (order independent) sits between them with no reordering.  Shared
+// memory bandwidth is what the transforms of 8 or more bins per CTA run
+// into, so there is one exchange through it per transform, and the twiddles
+// of the short transforms stay in registers.  At 1024 pulses Q = 1 and both
+// transforms share one copy of the code (conj-forward-conj), which keeps the
+// kernel within the instruction cache.
+//
+// Per iteration: each CTA sums conj(g) .* IFFT(T |T|) / M over its bins and
+// sends slice q of the sums to CTA q; CTA r adds the CL partials of its rows
+// in a fixed tree, normalises and sends the new phase to every CTA.  Both
+// messages are asynchronous stores into distributed shared memory that
+// count their bytes on the receiver's mbarrier: one one-way latency each,
+// where a cluster barrier also waits for the answer.  A receiver's buffer is
+// free again when its answer has come back, so one copy of each suffices.
+// The entropy of the selected bins, E = ln S1 - ln 2 * S2/S1 with
+// S1 = sum |T|^2, S2 = sum |T|^2 log2 |T|^2, comes out of the same epilogue
+// and drives the optional stop criterion (iterations that need it take a
+// cluster barrier more).
+//
+// Bound by latency: at 8 bins per CTA and 256 pulses an iteration is ~2700
+// clocks of transforms and ~2000 of reduction and messages.  Per iteration
+// (U = 64; team transforms with block barriers, gathers by remote loads and
+// two cluster barriers before -> now): 128 pulses 5.4 -> 2.1 us (4 CTAs),
+// 256 pulses 6.2 -> 2.3 (8 CTAs), 512 pulses 8.1 -> 3.4 (16 CTAs), 1024 pulses
+// 6.1 -> 5.2 (16 CTAs).  Two warps per bin (16 elements per lane, two tile
+// exchanges) measured 5.8 us at 1024 and 3.8 us at 512 pulses.
 // ---------------------------------------------------------------------------
 template <int M>
 struct AFC {
-    static constexpr int T = M / 16;
-    static constexpr int TEAMS = 4096 / M;     // 256 threads per CTA
-    static constexpr int THREADS = TEAMS * T;  // (two fused FFTs need ~255 registers: one CTA per SM)
-    static constexpr int NSLOT = 4;            // cached columns per CTA: 16384 / M
-    using Tw = TwShared<M, false, true>;       // two-level twiddles (80 entries at M = 1024)
-    // phase copy + FFT scratch (also holds P and the reduction buffer between
-    // sweeps) + column cache + twiddles: ~171 KB at M = 1024
+    static constexpr int P = M >= 1024 ? 32 : M == 512 ? 16 : 8;   // elements per lane
+    static constexpr int L = M / P;                                // lanes per bin
+    static constexpr int Q = L / P;
+    static constexpr int BW = 32 / L;                              // bins per warp
+    static constexpr int WARPS = 8;
+    static constexpr int THREADS = WARPS * 32;
+    static constexpr int BINS = WARPS * BW;                        // bins per round
+    static constexpr int CTAS = M >= 512 ? 1 : 2;                  // per SM (registers)
+    static constexpr int S1 = L + Q;   // tile row stride: both directions free of bank conflicts
+    static constexpr int TILE = P * S1;                            // per bin; also its M partial sums
+    static constexpr int NSLOT = 2;                                // cached rounds
+    static constexpr int BUF = M + 256;                            // [CL][M / CL + pad]
     static constexpr size_t SMEM_F2 =
-        (size_t)M + (size_t)TEAMS * FFTShape<M>::SMEM + (size_t)NSLOT * TEAMS * M + Tw::kEntries;
+        (size_t)M + BUF + (size_t)BINS * TILE + (size_t)NSLOT * BINS * M + (size_t)M + (size_t)P * Q;
     static constexpr size_t SMEM = SMEM_F2 * sizeof(float2) + 64 * sizeof(double);
-    static constexpr int PR = (M + THREADS - 1) / THREADS;   // partial-sum rows per thread
+    static_assert(TILE >= M && TILE % 2 == 0 && BUF % 2 == 0, "the tile also holds the bin's partial sums");
+    static_assert(P * L == M && P * Q == L && Q <= 4, "exchange pattern");
+    static_assert(SMEM <= 227 * 1024, "shared memory");
 };
 
 struct AFFrame {
@@ -480,9 +510,145 @@ struct AFFrame {
     float2* alt;           // [M] learned start phase in, the learned leg's final phase
                            // out (warm start), or null
     float2* gcol;          // [U][M] scratch: contiguous copy of the bin columns
+    unsigned* err;         // set when a message between the CTAs does not arrive
 };
 
-// With a learned start (AFFrame::alt), both cluster engines run two legs: the
+// The DFT over q (q = lane mod Q) of the elements c = 0..P-1 that Q
+// neighbouring lanes hold, as radix-2 steps: in a step lanes l and l ^ B keep
+// one half of the elements each, so every lane ends with P outputs.  The
+// lane with the bit set gets differences with the opposite sign; T |T| is
+// odd in T and the mirrored inverse undoes the sign, so it is not corrected.
+// step: v[2e], v[2e+1] -> v[2e] = kept + received, v[2e+1] = kept - received.
+template <int P, int B>
+__device__ __forceinline__ void cross_step(float2* v, bool hi)
+{
+#pragma unroll
+    for (int e = 0; e < P / 2; ++e) {
+        const float2 send = hi ? v[2 * e] : v[2 * e + 1], keep = hi ? v[2 * e + 1] : v[2 * e];
+        float2 got;
+        got.x = __shfl_xor_sync(0xffffffffu, send.x, B);
+        got.y = __shfl_xor_sync(0xffffffffu, send.y, B);
+        v[2 * e] = cadd(keep, got);
+        v[2 * e + 1] = csub(keep, got);
+    }
+}
+// The mirror image: kept = v[2e] + v[2e+1], the difference goes back.
+template <int P, int B>
+__device__ __forceinline__ void cross_step_back(float2* v, bool hi)
+{
+#pragma unroll
+    for (int e = 0; e < P / 2; ++e) {
+        const float2 keep = cadd(v[2 * e], v[2 * e + 1]), send = csub(v[2 * e], v[2 * e + 1]);
+        float2 got;
+        got.x = __shfl_xor_sync(0xffffffffu, send.x, B);
+        got.y = __shfl_xor_sync(0xffffffffu, send.y, B);
+        v[2 * e] = hi ? got : keep;
+        v[2 * e + 1] = hi ? keep : got;
+    }
+}
+template <int P, int Q>
+struct AfCross {
+    __device__ __forceinline__ static void forward(float2* v, int q)
+    {
+        if constexpr (Q == 2) {
+            cross_step<P, 1>(v, q & 1);
+        } else {
+            cross_step<P, 2>(v, q & 2);   // d0 = 0 in even registers, 1 in odd ones
+            float2 t[P];
+#pragma unroll
+            for (int e = 0; e < P / 2; ++e) {   // W_4^(q0 d0), then pair equal d0
+                const float2 x = v[2 * e + 1];
+                t[e] = v[2 * e];
+                t[P / 2 + e] = (q & 1) ? make_float2(x.y, -x.x) : x;
+            }
+            cross_step<P, 1>(t, q & 1);
+#pragma unroll
+            for (int e = 0; e < P; ++e) v[e] = t[e];
+        }
+    }
+    __device__ __forceinline__ static void inverse(float2* v, int q)
+    {
+        if constexpr (Q == 2) {
+            cross_step_back<P, 1>(v, q & 1);
+        } else {
+            cross_step_back<P, 1>(v, q & 1);
+            float2 t[P];
+#pragma unroll
+            for (int e = 0; e < P / 2; ++e) {
+                const float2 x = v[P / 2 + e];
+                t[2 * e] = v[e];
+                t[2 * e + 1] = (q & 1) ? make_float2(-x.y, x.x) : x;
+            }
+            cross_step_back<P, 2>(t, q & 2);
+#pragma unroll
+            for (int e = 0; e < P; ++e) v[e] = t[e];
+        }
+    }
+};
+
+// One mbarrier per message direction, one arrival (the receiver's own
+// expect_tx) and the message's bytes per phase.  Waits are bounded: one that
+// runs out sets *err and `dead`, after which no wait of the CTA waits again
+// and the kernel runs to its end (the host reports the frame as failed).
+constexpr unsigned kMsgWaitLimit = 1u << 20;
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank)
+{
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void msg_init(uint64_t* bar)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bar)) : "memory");
+}
+__device__ __forceinline__ void msg_expect(uint64_t* bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void msg_send(uint32_t dst, uint32_t bar, float2 a)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "f"(a.x), "f"(a.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void msg_send2(uint32_t dst, uint32_t bar, float2 a, float2 b)
+{
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                 "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void msg_wait(uint64_t* bar, uint32_t parity, volatile int* dead, unsigned* err)
+{
+    for (unsigned i = 0; i < kMsgWaitLimit; ++i) {
+        uint32_t done;
+        asm volatile("{\n .reg .pred p;\n"
+                     " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                     " selp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(done)
+                     : "r"(smem_u32(bar)), "r"(parity)
+                     : "memory");
+        if (done) return;
+        if (*dead) return;
+    }
+    *dead = 1;
+    atomicOr(err, 1u);
+}
+
+// T -> T |T|; an exact zero stays zero.
+__device__ __forceinline__ float2 times_abs(float2 v, bool ent, float& s1, float& s2)
+{
+    const float p = v.x * v.x + v.y * v.y;
+    if (ent) {
+        s1 += p;
+        if (p > 0.0f) s2 += p * __log2f(p);
+    }
+    const float a = p > 0.0f ? p * rsqrtf(p) : 0.0f;
+    return make_float2(v.x * a, v.y * a);
+}
+
+// With a learned start (AFFrame::alt) the engine runs two legs: the
 // autofocus from the learned start until the stop criterion (`tol`), then the
 // plain autofocus, the reference's algorithm (Doppler-tracking start, `iters`
 // updates, no stop criterion).  Both final phases are returned (alt, phase);
@@ -490,390 +656,214 @@ struct AFFrame {
 // so a frame on which the learned start ends worse reverts to the plain
 // result.  (The entropy of the selected bins cannot judge: it ignores a
 // linear phase, a Doppler shift of the image, which MTRC does not.)
-
+//
+// A CTA keeps NSLOT rounds of its bins in shared memory; when it has more,
+// the others are read from gcol, a contiguous copy of the gathered columns
+// ([U][M], written by the loading lanes themselves on entry), and successive
+// sweeps alternate direction so that the NSLOT rounds left in shared memory
+// by one sweep are the first of the next.
 template <int M>
-__global__ void __launch_bounds__(AFC<M>::THREADS, 1)
+__global__ void __launch_bounds__(AFC<M>::THREADS, AFC<M>::CTAS)
 k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
 {
     namespace cg = cooperative_groups;
     using A = AFC<M>;
-    using F = FFTShape<M>;
-    using TwA = typename A::Tw;
+    constexpr int P = A::P, L = A::L, Q = A::Q;
     cg::cluster_group cl = cg::this_cluster();
     const int CL = (int)cl.num_blocks();
     const int r = (int)cl.block_rank();
     extern __shared__ float4 dyn_smem[];
-    float2* ph = reinterpret_cast<float2*>(dyn_smem);   // [M]
-    float2* smb = ph + M;                                // [TEAMS][SMEM]; between sweeps: P [M], buf
-    float2* P = smb;
-    float2* cache = smb + A::TEAMS * F::SMEM;            // [NSLOT][TEAMS][M]
-    float2* twt = cache + (size_t)A::NSLOT * A::TEAMS * M;   // twiddle table
-    double* red = reinterpret_cast<double*>(twt + TwA::kEntries);   // [64]
-    const TwA tws{twt};
-    const int tid = threadIdx.x;
-    TwA::fill(twt, tw, tid, A::THREADS);
-    const int team = tid / F::T, lt = tid % F::T;
-    const int lane = tid & 31, warp = tid >> 5;
-    const int U = f.fdec[1];
-    const int bpc = (U + CL - 1) / CL;
-    const int b0 = r * bpc;
-    const int nb = max(0, min(bpc, U - b0));
-    const int nch = (nb + A::TEAMS - 1) / A::TEAMS;
-    const bool reload = nch > A::NSLOT;
-    float2* sm = smb + team * F::SMEM;
-
-    auto load_chunk = [&](int j, int slot) {
-        const int t = j * A::TEAMS + team;
-        float2* g = cache + ((size_t)slot * A::TEAMS + team) * M;
-        if (t < nb) {
-            const int b = f.bins[b0 + t];
-            for (int m = lt; m < M; m += F::T) g[m] = f.cut[(size_t)m * C + b];
-        }
-    };
-    for (int m = tid; m < M; m += A::THREADS) ph[m] = f.phase[m];
-    for (int j = 0; j < min(nch, A::NSLOT); ++j) load_chunk(j, j);
-    __syncthreads();
-
-    const float invM = 1.0f / (float)M;
-    const int rows = M / CL;
-
-    // One sweep over this CTA's bins with the phase in ph: entropy sums
-    // (s1, s2, only when `ent`) and, when `full`, the partial row sums of the
-    // update, accumulated in registers and left in P (the start of the FFT
-    // scratch) for the cluster reduction.
-    auto sweep = [&](bool full, bool ent, float& s1, float& s2) {
-        float2 pacc[A::PR];
-#pragma unroll
-        for (int k = 0; k < A::PR; ++k) pacc[k] = make_float2(0.0f, 0.0f);
-#pragma unroll 1
-        for (int j = 0; j < nch; ++j) {
-            const int slot = j < A::NSLOT ? j : A::NSLOT - 1;
-            if (reload && j >= A::NSLOT - 1) {
-                __syncthreads();
-                load_chunk(j, slot);
-            }
-            __syncthreads();
-            const float2* g = cache + ((size_t)slot * A::TEAMS + team) * M;
-            const bool valid = j * A::TEAMS + team < nb;
-            team_fft<M, false>([&](int i) { return cmul(ph[i], g[i]); },
-                               [&](int i, float2 v, int) {
-                                   const float p = v.x * v.x + v.y * v.y;
-                                   if (ent) {
-                                       s1 += p;
-                                       if (p > 0.0f) s2 += p * __log2f(p);
-                                   }
-                                   sm[fpad(i)] = cscale(v, sqrtf(p));
-                               },
-                               sm, lt, tws, valid);
-            if (!full) continue;
-            team_fft<M, true>([&](int i) { return sm[fpad(i)]; },
-                              [&](int i, float2 v, int) { sm[fpad(i)] = cmulc(g[i], cscale(v, invM)); }, sm, lt,
-                              tws, valid);
-            const int nt = min(A::TEAMS, nb - j * A::TEAMS);
-#pragma unroll
-            for (int k = 0; k < A::PR; ++k) {
-                const int m = tid + k * A::THREADS;
-                if (m < M)
-                    for (int t = 0; t < nt; ++t) {
-                        const float2 q = smb[t * F::SMEM + fpad(m)];
-                        pacc[k].x += q.x;
-                        pacc[k].y += q.y;
-                    }
-            }
-        }
-        if (full) {
-            __syncthreads();   // every team is done with the scratch
-#pragma unroll
-            for (int k = 0; k < A::PR; ++k) {
-                const int m = tid + k * A::THREADS;
-                if (m < M) P[m] = pacc[k];
-            }
-        }
-    };
-
-    // Entropy of the selected bins from the per-thread sums of one sweep:
-    // float per warp, double per CTA (red[32..33]) and per cluster, by thread
-    // 0 of every CTA in the same order (FP64 is slow on this part).  The
-    // cluster barrier inside publishes red[32..33]; the caller's next cluster
-    // barrier must come before they are rewritten.  Returns the value in
-    // thread 0.
-    auto entropy_sums = [&](float s1, float s2) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-            s2 += __shfl_xor_sync(0xffffffffu, s2, o);
-        }
-        if (lane == 0) {
-            red[warp] = s1;
-            red[16 + warp] = s2;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double a1 = 0.0, a2 = 0.0;
-            for (int w = 0; w < A::THREADS / 32; ++w) {
-                a1 += red[w];
-                a2 += red[16 + w];
-            }
-            red[32] = a1;
-            red[33] = a2;
-        }
-        cl.sync();
-        float E = 0.0f;
-        if (tid == 0) {
-            double S1 = 0.0, S2 = 0.0;
-            for (int q = 0; q < CL; ++q) {
-                const double* rr = cl.map_shared_rank(red, q);
-                S1 += rr[32];
-                S2 += rr[33];
-            }
-            E = logf((float)S1) - kLn2 * (float)S2 / (float)S1;
-        }
-        return E;
-    };
-
-    // One autofocus run from the phase in ph: up to `iters` updates, fewer
-    // when the stop criterion ends it.  Returns (in thread 0) the entropy at
-    // the last evaluated phase or, with want_final, of the final phase (one
-    // more entropy sweep when all `iters` updates were applied).
-    auto leg = [&](bool want_final, float ltol, int& used) -> float {
-        float e_prev = 0.0f, e_last = 0.0f;   // meaningful in thread 0
-        bool stopped = false;
-        used = iters;
-#pragma unroll 1
-        for (int it = 0; it < iters; ++it) {
-            // the entropy is needed by the stop criterion, and for the trace at
-            // the last iteration; elsewhere its logarithms are skipped
-            const bool check = ltol > 0.0f && it % kStopEvery == 0;
-            const bool need_e = check || it == iters - 1;
-            float s1 = 0.0f, s2 = 0.0f;
-            sweep(true, need_e, s1, s2);
-            const float E = entropy_sums(s1, s2);
-            if (tid == 0) {
-                bool stop = false;
-                if (need_e) {
-                    if (check) {
-                        stop = it > 0 && fabsf(E - e_prev) <= (float)kStopEvery * ltol * fabsf(E);
-                        e_prev = E;
-                    }
-                    e_last = E;
-                }
-                red[40] = stop ? 1.0 : 0.0;
-            }
-            // This CTA's rows [r*rows, (r+1)*rows) of every CTA's partial sums,
-            // gathered with independent remote loads into buf[q][row] (behind P).
-            float2* buf = smb + M;
-            for (int idx = tid; idx < CL * rows; idx += A::THREADS) {
-                const int q = idx / rows, ml = idx - q * rows;
-                buf[idx] = cl.map_shared_rank(P, q)[r * rows + ml];
-            }
-            __syncthreads();
-            const bool stop = red[40] != 0.0;
-            if (!stop) {
-                for (int ml = tid; ml < rows; ml += A::THREADS) {
-                    float2 s = make_float2(0.0f, 0.0f);
-                    for (int q = 0; q < CL; ++q) {
-                        const float2 v = buf[q * rows + ml];
-                        s.x += v.x;
-                        s.y += v.y;
-                    }
-                    const float a = sqrtf(s.x * s.x + s.y * s.y);
-                    buf[CL * rows + ml] = make_float2(s.x / a, s.y / a);
-                }
-                __syncthreads();
-                for (int idx = tid; idx < CL * rows; idx += A::THREADS) {
-                    const int q = idx / rows, ml = idx - q * rows;
-                    cl.map_shared_rank(ph, q)[r * rows + ml] = buf[CL * rows + ml];
-                }
-            }
-            cl.sync();
-            if (stop) {
-                used = it;
-                stopped = true;
-                break;
-            }
-        }
-        if (want_final && !stopped) {
-            float s1 = 0.0f, s2 = 0.0f;
-            sweep(false, true, s1, s2);
-            const float E = entropy_sums(s1, s2);
-            if (tid == 0) e_last = E;
-            cl.sync();   // red[32..33] are read remotely before a later sweep rewrites them
-        }
-        return e_last;
-    };
-
-    if (!f.alt) {
-        int used;
-        const float e = leg(false, tol, used);
-        for (int m = r * rows + tid; m < (r + 1) * rows; m += A::THREADS) f.phase[m] = ph[m];
-        if (r == 0 && tid == 0 && f.stat) {
-            f.stat[0] = used;
-            f.stat[1] = __float_as_int(e);
-        }
-        return;
-    }
-    // the learned leg, then the plain leg (see AFFrame)
-    __syncthreads();
-    for (int m = tid; m < M; m += A::THREADS) ph[m] = f.alt[m];
-    __syncthreads();
-    int used_l, used_d;
-    const float e_l = leg(false, tol, used_l);
-    for (int m = r * rows + tid; m < (r + 1) * rows; m += A::THREADS) f.alt[m] = ph[m];
-    __syncthreads();
-    for (int m = tid; m < M; m += A::THREADS) ph[m] = f.phase[m];
-    __syncthreads();
-    const float e_d = leg(false, 0.0f, used_d);
-    for (int m = r * rows + tid; m < (r + 1) * rows; m += A::THREADS) f.phase[m] = ph[m];
-    if (r == 0 && tid == 0 && f.stat) {
-        f.stat[0] = used_l + used_d;
-        f.stat[1] = __float_as_int(e_d);
-        f.stat[2] = 0;
-        f.stat[3] = __float_as_int(e_d);
-        f.stat[4] = __float_as_int(e_l);
-        f.stat[5] = used_d;
-        f.stat[6] = used_l;
-    }
-}
-
-// ---------------------------------------------------------------------------
-// k_af_cluster for M = 1024 on warp-level FFTs (warp_fft1024): one warp per
-// bin, 8 bins per round per CTA.  Element m of a bin lives in lane m % 32,
-// register m / 32 through the forward transform, the T |T| epilogue and the
-// inverse transform (conj-forward-conj); the transposes go through the
-// warp's own tile, so no block barrier sits inside a sweep.  Per-warp partial
-// row sums accumulate in registers across rounds and are reduced over the
-// CTA's warps in fixed order; the cluster reduction, stop criterion and the
-// choice of start are those of k_af_cluster.
-// ---------------------------------------------------------------------------
-struct AFW {
-    static constexpr int M = 1024;
-    static constexpr int WARPS = 8;
-    static constexpr int THREADS = WARPS * 32;
-    static constexpr int TILE = 32 * 33;       // per-warp transpose tile (float2)
-    static constexpr int NSLOT = 2;            // cached rounds: 16 bins per CTA
-    static constexpr size_t SMEM_F2 = (size_t)M + (size_t)WARPS * TILE + (size_t)NSLOT * WARPS * M + M;
-    static constexpr size_t SMEM = SMEM_F2 * sizeof(float2) + 64 * sizeof(double);
-};
-
-// Each warp keeps NSLOT of its bins in shared memory; when the CTA has more,
-// the others are read from gcol, a contiguous copy of the
-// gathered columns ([U][M], written by the loading warp itself on entry), and
-// successive sweeps alternate direction so that the NSLOT rounds left in
-// shared memory by one sweep are the first of the next.
-__global__ void __launch_bounds__(AFW::THREADS, 1)
-k_af_cluster_w1024(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
-{
-    namespace cg = cooperative_groups;
-    constexpr int M = AFW::M;
-    cg::cluster_group cl = cg::this_cluster();
-    const int CL = (int)cl.num_blocks();
-    const int r = (int)cl.block_rank();
-    extern __shared__ float4 dyn_smem[];
+    __shared__ __align__(8) uint64_t bar_part, bar_ph;          // partial sums, phase slices arrived
+    __shared__ int dead;
     float2* ph = reinterpret_cast<float2*>(dyn_smem);          // [M]
-    float2* tiles = ph + M;                                     // [WARPS][TILE]; between sweeps P, buf
-    float2* cache = tiles + AFW::WARPS * AFW::TILE;             // [NSLOT][WARPS][M]
-    float2* TWL = cache + (size_t)AFW::NSLOT * AFW::WARPS * M;  // [32][32] W^(lane k)
-    double* red = reinterpret_cast<double*>(TWL + M);           // [64]
-    float2* P = tiles;
+    float2* buf = ph + M;                                       // [CL][bs] partial sums of this CTA's rows
+    float2* tiles = buf + A::BUF;                               // [BINS][TILE]
+    float2* cache = tiles + A::BINS * A::TILE;                  // [NSLOT][BINS][M]
+    float2* T1 = cache + (size_t)A::NSLOT * A::BINS * M;        // [P][L] W_M^(l k)
+    float2* T2 = T1 + M;                                        // [P][Q] W_L^(q c)
+    double* red = reinterpret_cast<double*>(T2 + P * Q);        // [64]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (int i = tid; i < M; i += AFW::THREADS) TWL[i] = tw[(i >> 5) * (i & 31) * (kTwN / M)];
-    float2* tile = tiles + warp * AFW::TILE;
+    const int slot = tid / L, l = tid & (L - 1);                // bin within a round, lane within the bin
+    const int k1 = l / Q, q = l & (Q - 1);
+    if (tid == 0) {
+        dead = 0;
+        msg_init(&bar_part);
+        msg_init(&bar_ph);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int i = tid; i < M; i += A::THREADS) T1[i] = tw[(i / L) * (i & (L - 1)) * (kTwN / M)];
+    for (int i = tid; i < P * Q; i += A::THREADS) T2[i] = tw[(i / Q) * (i & (Q - 1)) * (kTwN / L)];
+    float2* ta = tiles + slot * A::TILE;
     const int U = f.fdec[1];
     const int bpc = (U + CL - 1) / CL;
     const int b0 = r * bpc;
     const int nb = max(0, min(bpc, U - b0));
-    const int nrd = (nb + AFW::WARPS - 1) / AFW::WARPS;
-    const bool reload = nrd > AFW::NSLOT;
-    float2* gw = f.gcol + (size_t)(b0 + warp) * M;   // this warp's bin of round 0
+    const int nrd = (nb + A::BINS - 1) / A::BINS;
+    const int nact = min(A::BINS, nb);                          // bins with partial sums
+    const bool reload = nrd > A::NSLOT;
+    float2* gw = f.gcol + (size_t)(b0 + slot) * M;              // its column of round 0
 
-    for (int m = tid; m < M; m += AFW::THREADS) ph[m] = f.phase[m];
-    // every bin of this warp: cached rounds into their slot, all rounds into
-    // gcol when some must be re-read
+    for (int m = tid; m < M; m += A::THREADS) ph[m] = f.phase[m];
     for (int j = 0; j < nrd; ++j) {
-        const int t = j * AFW::WARPS + warp;
-        if (t >= nb || (j >= AFW::NSLOT && !reload)) continue;
+        const int t = j * A::BINS + slot;
+        if (t >= nb || (j >= A::NSLOT && !reload)) continue;
         const int b = f.bins[b0 + t];
-        float2* g = cache + ((size_t)(j % AFW::NSLOT) * AFW::WARPS + warp) * M;
-        float2* gg = gw + (size_t)j * AFW::WARPS * M;
-        for (int m = lane; m < M; m += 32) {
+        float2* g = cache + ((size_t)(j % A::NSLOT) * A::BINS + slot) * M;
+        float2* gg = gw + (size_t)j * A::BINS * M;
+#pragma unroll 4
+        for (int i = 0; i < P; ++i) {
+            const int m = l + L * i;
             const float2 x = f.cut[(size_t)m * C + b];
-            if (j < AFW::NSLOT) g[m] = x;
+            if (j < A::NSLOT) g[m] = x;
             if (reload) gg[m] = x;
         }
     }
-    __syncthreads();
+    cl.sync();   // every CTA of the cluster runs and has its mbarriers: messages may be sent
 
     const float invM = 1.0f / (float)M;
     const int rows = M / CL;
-    int nsweep = 0;
-
-    // One sweep with the phase in ph; see k_af_cluster.
-    auto sweep = [&](bool full, bool ent, float& s1, float& s2) {
-        float2 pacc[32];
+    const int lg_rows = 31 - __clz(rows);
+    // threads per row of the cluster reduction, and the row stride of buf that
+    // keeps their reads in different banks
+    const int tpr = min(CL, A::THREADS / rows);
+    const int bs = rows + 16 / tpr + ((16 / tpr) & 1);
+    // twiddles of the short transforms in registers
+    constexpr bool kRegTw = P <= 8;
+    float2 w1[kRegTw ? P : 1], w2[kRegTw ? P : 1];
+    if constexpr (kRegTw) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) pacc[k] = make_float2(0.0f, 0.0f);
+        for (int k = 0; k < P; ++k) {
+            w1[k] = T1[k * L + l];
+            w2[k] = T2[k * Q + q];
+        }
+    }
+    auto t1 = [&](int k) {
+        if constexpr (kRegTw) return w1[k];
+        else return T1[k * L + l];
+    };
+    auto t2 = [&](int c) {
+        if constexpr (kRegTw) return w2[c];
+        else return T2[c * Q + q];
+    };
+    int nsweep = 0;
+    uint32_t par = 0;   // phase parity of both mbarriers: bit 0 bar_part, bit 1 bar_ph
+
+    // One sweep over this CTA's bins with the phase in ph: entropy sums
+    // (s1, s2, only when `ent`) and the partial row sums of the update, sent
+    // to the CTAs that own the rows.
+    auto sweep = [&](bool ent, float& s1, float& s2) {
+        float2 pacc[P];
+#pragma unroll
+        for (int i = 0; i < P; ++i) pacc[i] = make_float2(0.0f, 0.0f);
         const bool back = (nsweep++ & 1) != 0;
 #pragma unroll 1
         for (int jj = 0; jj < nrd; ++jj) {
             const int j = back ? nrd - 1 - jj : jj;
-            if (j * AFW::WARPS + warp >= nb) continue;   // warp-uniform; no block barrier inside
-            float2* g = cache + ((size_t)(j % AFW::NSLOT) * AFW::WARPS + warp) * M;
-            if (jj >= AFW::NSLOT) {   // only when reload: read the copy in gcol
-                const float4* src = reinterpret_cast<const float4*>(gw + (size_t)j * AFW::WARPS * M);
+            if (j * A::BINS + warp * A::BW >= nb) continue;   // warp-uniform; no block barrier inside
+            const bool valid = A::BW == 1 || j * A::BINS + slot < nb;
+            float2* g = cache + ((size_t)(j % A::NSLOT) * A::BINS + slot) * M;
+            __syncwarp();   // the slot and the tile of the previous round are read
+            if (jj >= A::NSLOT && valid) {   // only when reload: read the copy in gcol
+                const float4* src = reinterpret_cast<const float4*>(gw + (size_t)j * A::BINS * M);
                 float4* dst = reinterpret_cast<float4*>(g);
 #pragma unroll 4
-                for (int i = lane; i < M / 2; i += 32) dst[i] = src[i];
-                __syncwarp();
+                for (int i = l; i < M / 2; i += L) dst[i] = src[i];
             }
-            float2 v[32];
+            __syncwarp();
+            float2 v[P];
 #pragma unroll
-            for (int k = 0; k < 32; ++k) v[k] = cmul(ph[lane + 32 * k], g[lane + 32 * k]);
-            // pass 0: T = FFT(phase * g); pass 1: conj(IFFT(T |T|)) * M as the
-            // forward FFT of conj(T |T|).  One copy of the transform's code
-            // (a loop, not unrolled) keeps the kernel within the instruction
-            // cache.
+            for (int i = 0; i < P; ++i)
+                v[i] = valid ? cmul(ph[l + L * i], g[l + L * i]) : make_float2(0.0f, 0.0f);
+            if constexpr (Q == 1) {
+                // pass 0: T = FFT(phase * g); pass 1: conj(IFFT(T |T|)) * M as
+                // the forward FFT of conj(T |T|)
 #pragma unroll 1
-            for (int pass = 0; pass < (full ? 2 : 1); ++pass) {
-                warp_fft1024(v, lane, tile, TWL);
-                if (pass == 0) {
+                for (int pass = 0; pass < 2; ++pass) {
+                    // two DFT steps sharing one copy of the code
+#pragma unroll 1
+                    for (int step = 0;; ++step) {
+                        dft32_reg(v);
+                        if (step == 1) break;
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) {
-                        const float p = v[k].x * v[k].x + v[k].y * v[k].y;
-                        if (ent) {
-                            s1 += p;
-                            if (p > 0.0f) s2 += p * __log2f(p);
+                        for (int k = 1; k < P; ++k) v[k] = cmul(v[k], T1[k * L + l]);
+#pragma unroll
+                        for (int k = 0; k < P; ++k) ta[l * A::S1 + k] = v[k];
+                        __syncwarp();
+#pragma unroll
+                        for (int n = 0; n < P; ++n) v[n] = ta[n * A::S1 + l];
+                        __syncwarp();
+                    }
+                    if (pass == 0) {
+#pragma unroll
+                        for (int i = 0; i < P; ++i) v[i] = conjf2(times_abs(v[i], ent, s1, s2));
+                    } else {
+                        // conj(g) conj(v) = conj(g v): the conjugate is applied once per sweep
+#pragma unroll
+                        for (int i = 0; i < P; ++i) {
+                            const float2 x = g[l + L * i];
+                            pacc[i].x = fmaf(x.x, v[i].x, fmaf(-x.y, v[i].y, pacc[i].x));
+                            pacc[i].y = fmaf(x.x, v[i].y, fmaf(x.y, v[i].x, pacc[i].y));
                         }
-                        const float a = p > 0.0f ? p * rsqrtf(p) : 0.0f;
-                        v[k] = make_float2(v[k].x * a, -v[k].y * a);   // conj(T |T|)
                     }
-                } else {
-                    // conj(g) conj(v) / M = conj(g v) / M: g v accumulates
-                    // here, the conjugate and 1/M are applied once per sweep
+                }
+            } else {
+                dft_reg<P, false>(v);
 #pragma unroll
-                    for (int k = 0; k < 32; ++k) {
-                        const float2 q = g[lane + 32 * k];
-                        pacc[k].x = fmaf(q.x, v[k].x, fmaf(-q.y, v[k].y, pacc[k].x));
-                        pacc[k].y = fmaf(q.x, v[k].y, fmaf(q.y, v[k].x, pacc[k].y));
+                for (int k = 1; k < P; ++k) v[k] = cmul(v[k], t1(k));
+#pragma unroll
+                for (int k = 0; k < P; ++k) ta[k * A::S1 + l] = v[k];
+                __syncwarp();
+#pragma unroll
+                for (int b = 0; b < P; ++b) v[b] = ta[k1 * A::S1 + q + Q * b];
+                dft_reg<P, false>(v);
+#pragma unroll
+                for (int c = 1; c < P; ++c) v[c] = cmul(v[c], t2(c));
+                AfCross<P, Q>::forward(v, q);
+#pragma unroll
+                for (int i = 0; i < P; ++i) v[i] = times_abs(v[i], ent, s1, s2);
+                AfCross<P, Q>::inverse(v, q);
+#pragma unroll
+                for (int c = 1; c < P; ++c) v[c] = cmulc(t2(c), v[c]);
+                dft_reg<P, true>(v);
+                __syncwarp();   // every lane has read the tile
+#pragma unroll
+                for (int b = 0; b < P; ++b) ta[k1 * A::S1 + q + Q * b] = v[b];
+                __syncwarp();
+#pragma unroll
+                for (int k = 0; k < P; ++k) v[k] = ta[k * A::S1 + l];
+#pragma unroll
+                for (int k = 1; k < P; ++k) v[k] = cmulc(t1(k), v[k]);
+                dft_reg<P, true>(v);
+                if (valid) {
+#pragma unroll
+                    for (int i = 0; i < P; ++i) {
+                        const float2 x = g[l + L * i];   // conj(x) v
+                        pacc[i].x = fmaf(x.x, v[i].x, fmaf(x.y, v[i].y, pacc[i].x));
+                        pacc[i].y = fmaf(x.x, v[i].y, fmaf(-x.y, v[i].x, pacc[i].y));
                     }
                 }
             }
-            __syncwarp();   // slot reuse by a later reload
         }
-        if (full) {
-            __syncthreads();   // every warp is done with its tile
+        // the bins' sums to the rows' owners, two rows per message
+        __syncwarp();   // the tile is read
+        if (slot < nact) {
+            const float sy = Q == 1 ? -invM : invM;
 #pragma unroll
-            for (int k = 0; k < 32; ++k) tile[lane + 32 * k] = make_float2(pacc[k].x * invM, -pacc[k].y * invM);
-            __syncthreads();
-            for (int m = tid; m < M; m += AFW::THREADS) {
-                float2 s = tiles[m];
+            for (int i = 0; i < P; ++i) ta[l + L * i] = make_float2(pacc[i].x * invM, pacc[i].y * sy);
+        }
+        __syncthreads();
+        for (int m = 2 * tid; m < M; m += 2 * A::THREADS) {
+            float2 a = make_float2(0.0f, 0.0f), b = a;
 #pragma unroll
-                for (int w = 1; w < AFW::WARPS; ++w) {
-                    const float2 q = tiles[w * AFW::TILE + m];
-                    s.x += q.x;
-                    s.y += q.y;
+            for (int x = 0; x < A::BINS; ++x)
+                if (x < nact) {
+                    const float4 t = *reinterpret_cast<const float4*>(&tiles[x * A::TILE + m]);
+                    a = cadd(a, make_float2(t.x, t.y));
+                    b = cadd(b, make_float2(t.z, t.w));
                 }
-                P[m] = s;
-            }
+            const int to = m >> lg_rows;
+            msg_send2(cluster_addr(smem_u32(&buf[r * bs + (m & (rows - 1))]), to), cluster_addr(smem_u32(&bar_part), to),
+                      a, b);
         }
     };
 
@@ -895,7 +885,7 @@ k_af_cluster_w1024(AFFrame f, int iters, float tol, const float2* __restrict__ t
         __syncthreads();
         if (tid == 0) {
             double a1 = 0.0, a2 = 0.0;
-            for (int w = 0; w < AFW::WARPS; ++w) {
+            for (int w = 0; w < A::WARPS; ++w) {
                 a1 += red[w];
                 a2 += red[16 + w];
             }
@@ -918,114 +908,106 @@ k_af_cluster_w1024(AFFrame f, int iters, float tol, const float2* __restrict__ t
         return logf((float)S1) - kLn2 * (float)S2 / (float)S1;
     };
 
-    // One autofocus run from the phase in ph (see k_af_cluster): returns, in
-    // warp 0, the entropy at the last evaluated phase or, with want_final, of
-    // the final phase.
-    float2* buf = tiles + AFW::TILE;   // behind P (tile 0 holds P)
-    auto leg = [&](bool want_final, float ltol, int& used) -> float {
+    // One autofocus run from the phase in ph: up to `iters` updates, fewer
+    // when the stop criterion ends it.  Returns, in warp 0, the entropy at the
+    // last evaluated phase.
+    auto leg = [&](float ltol, int& used) -> float {
         float e_prev = 0.0f, e_last = 0.0f;   // meaningful in warp 0
-        bool stopped = false;
         used = iters;
-        int lg_rows = 0;
-        while ((1 << lg_rows) < rows) ++lg_rows;
 #pragma unroll 1
         for (int it = 0; it < iters; ++it) {
             // the entropy is needed by the stop criterion or for the last trace
             const bool check = ltol > 0.0f && it % kStopEvery == 0;
             const bool need_e = check || it == iters - 1;
             float s1 = 0.0f, s2 = 0.0f;
-            sweep(true, need_e, s1, s2);
-            if (need_e) entropy_part(s1, s2);
-            cl.sync();   // P and red[32..33] of every CTA are complete
-            if (warp == 0) {
-                bool stop = false;
-                if (need_e) {
+            sweep(need_e, s1, s2);
+            bool stop = false;
+            if (need_e) {
+                entropy_part(s1, s2);
+                cl.sync();   // red[32..33] of every CTA are complete
+                if (warp == 0) {
                     const float E = entropy_total();
                     if (check) {
                         stop = it > 0 && fabsf(E - e_prev) <= (float)kStopEvery * ltol * fabsf(E);
                         e_prev = E;
                     }
                     e_last = E;
-                }
-                if (lane == 0) red[40] = stop ? 1.0 : 0.0;
-            }
-            // this CTA's rows of the cluster sum: slice r of every CTA's P
-#pragma unroll
-            for (int i = 0; i < M / AFW::THREADS; ++i) {
-                const int idx = tid + i * AFW::THREADS;
-                const int q = idx >> lg_rows, ml = idx & (rows - 1);
-                buf[idx] = cl.map_shared_rank(P, q)[r * rows + ml];
-            }
-            __syncthreads();
-            const bool stop = red[40] != 0.0;
-            if (!stop) {
-                for (int ml = tid; ml < rows; ml += AFW::THREADS) {
-                    float2 s = make_float2(0.0f, 0.0f);
-                    for (int q = 0; q < CL; ++q) {
-                        const float2 v = buf[q * rows + ml];
-                        s.x += v.x;
-                        s.y += v.y;
-                    }
-                    const float a = sqrtf(s.x * s.x + s.y * s.y);
-                    buf[M + ml] = make_float2(s.x / a, s.y / a);
+                    if (lane == 0) red[40] = stop ? 1.0 : 0.0;
                 }
                 __syncthreads();
-#pragma unroll
-                for (int i = 0; i < M / AFW::THREADS; ++i) {
-                    const int idx = tid + i * AFW::THREADS;
-                    const int q = idx >> lg_rows, ml = idx & (rows - 1);
-                    cl.map_shared_rank(ph, q)[r * rows + ml] = buf[M + ml];
-                }
+                stop = red[40] != 0.0;
             }
-            cl.sync();
+            if (tid == 0) msg_expect(&bar_part, M * sizeof(float2));
+            msg_wait(&bar_part, par & 1, &dead, f.err);
+            par ^= 1;
             if (stop) {
+                cl.sync();   // every CTA has these messages: the next leg may send
                 used = it;
-                stopped = true;
                 break;
             }
-        }
-        if (want_final && !stopped) {
-            float s1 = 0.0f, s2 = 0.0f;
-            sweep(false, true, s1, s2);
-            entropy_part(s1, s2);
-            cl.sync();
-            if (warp == 0) e_last = entropy_total();
-            cl.sync();   // red[32..33] are read remotely before a later sweep rewrites them
+            // tpr neighbouring threads add a row's CL partial sums (fixed
+            // tree) and send its new phase to CL / tpr CTAs each
+            for (int idx = tid; idx < rows * tpr; idx += A::THREADS) {
+                const int part = idx & (tpr - 1), ml = idx / tpr;
+                float2 s = buf[part * bs + ml];
+                for (int x = part + tpr; x < CL; x += tpr) s = cadd(s, buf[x * bs + ml]);
+                for (int o = tpr >> 1; o > 0; o >>= 1) {
+                    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+                    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+                }
+                const float a = sqrtf(s.x * s.x + s.y * s.y);
+                s = make_float2(s.x / a, s.y / a);
+                for (int to = part; to < CL; to += tpr)
+                    msg_send(cluster_addr(smem_u32(&ph[r * rows + ml]), to), cluster_addr(smem_u32(&bar_ph), to), s);
+            }
+            if (tid == 0) msg_expect(&bar_ph, M * sizeof(float2));
+            msg_wait(&bar_ph, par >> 1, &dead, f.err);
+            par ^= 2;
         }
         return e_last;
     };
 
     if (!f.alt) {
         int used;
-        const float e = leg(false, tol, used);
-        for (int m = r * rows + tid; m < (r + 1) * rows; m += AFW::THREADS) f.phase[m] = ph[m];
+        const float e = leg(tol, used);
+        for (int m = r * rows + tid; m < (r + 1) * rows; m += A::THREADS) f.phase[m] = ph[m];
         if (r == 0 && tid == 0 && f.stat) {
             f.stat[0] = used;
             f.stat[1] = __float_as_int(e);
         }
+        cl.sync();   // no CTA leaves while another may still send to it
         return;
     }
-    // the learned leg, then the plain leg (see AFFrame)
-    __syncthreads();
-    for (int m = tid; m < M; m += AFW::THREADS) ph[m] = f.alt[m];
-    __syncthreads();
-    int used_l, used_d;
-    const float e_l = leg(false, tol, used_l);
-    for (int m = r * rows + tid; m < (r + 1) * rows; m += AFW::THREADS) f.alt[m] = ph[m];
-    __syncthreads();
-    for (int m = tid; m < M; m += AFW::THREADS) ph[m] = f.phase[m];
-    __syncthreads();
-    const float e_d = leg(false, 0.0f, used_d);
-    for (int m = r * rows + tid; m < (r + 1) * rows; m += AFW::THREADS) f.phase[m] = ph[m];
-    if (r == 0 && tid == 0 && f.stat) {
-        f.stat[0] = used_l + used_d;
-        f.stat[1] = __float_as_int(e_d);
-        f.stat[2] = 0;
-        f.stat[3] = __float_as_int(e_d);
-        f.stat[4] = __float_as_int(e_l);
-        f.stat[5] = used_d;
-        f.stat[6] = used_l;
+    // the learned leg, then the plain leg (one copy of the code)
+    int used[2];
+    float e[2];
+#pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+        float2* p = k == 0 ? f.alt : f.phase;
+        __syncthreads();
+        for (int m = tid; m < M; m += A::THREADS) ph[m] = p[m];
+        __syncthreads();
+        int u;
+        const float x = leg(k == 0 ? tol : 0.0f, u);
+        if (k == 0) {
+            used[0] = u;
+            e[0] = x;
+        } else {
+            used[1] = u;
+            e[1] = x;
+        }
+        for (int m = r * rows + tid; m < (r + 1) * rows; m += A::THREADS) p[m] = ph[m];
     }
+    if (r == 0 && tid == 0 && f.stat) {
+        f.stat[0] = used[0] + used[1];
+        f.stat[1] = __float_as_int(e[1]);
+        f.stat[2] = 0;
+        f.stat[3] = __float_as_int(e[1]);
+        f.stat[4] = __float_as_int(e[0]);
+        f.stat[5] = used[1];
+        f.stat[6] = used[0];
+    }
+    cl.sync();   // no CTA leaves while another may still send to it
 }
 
 // cut[m][c] *= phase[m]  (phase_adjustment.cu:324)
@@ -1056,32 +1038,17 @@ __global__ void k_af_apply2(float2* __restrict__ cut, const float2* __restrict__
 template <int M>
 static constexpr int af_cb() { return M >= 512 ? 8 : (M >= 256 ? 16 : 32); }
 
-// The cluster engine's kernel for M pulses: warp-level FFTs at M = 1024,
-// team FFTs otherwise.
-template <int M>
-struct AfEngine {
-    static constexpr bool kWarp = M == 1024;
-    static constexpr int THREADS = kWarp ? AFW::THREADS : AFC<M>::THREADS;
-    static constexpr size_t SMEM = kWarp ? AFW::SMEM : AFC<M>::SMEM;
-    using Fn = void (*)(AFFrame, int, float, const float2*);
-    static Fn kernel()
-    {
-        if constexpr (kWarp) return k_af_cluster_w1024;
-        else return k_af_cluster<M>;
-    }
-};
-
 // Cluster engine set-up (once per device): shared-memory limit, non-portable
 // cluster sizes, and the largest of 16/8/4 CTAs per cluster that can be
 // resident.  Returns that size, 0 if none, or a negative cudaError_t.
 template <int M>
 static int af_cluster_probe()
 {
-    using A = AfEngine<M>;
+    using A = AFC<M>;
     cudaError_t e;
-    if ((e = cudaFuncSetAttribute(A::kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A::SMEM)))
+    if ((e = cudaFuncSetAttribute(k_af_cluster<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A::SMEM)))
         return -(int)e;
-    if ((e = cudaFuncSetAttribute(A::kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) {
+    if ((e = cudaFuncSetAttribute(k_af_cluster<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) {
         (void)cudaGetLastError();
     }
     int best = 0;
@@ -1098,7 +1065,7 @@ static int af_cluster_probe()
         cfg.attrs = at;
         cfg.numAttrs = 1;
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, A::kernel(), &cfg) == cudaSuccess && n > 0) best = cl;
+        if (cudaOccupancyMaxActiveClusters(&n, k_af_cluster<M>, &cfg) == cudaSuccess && n > 0) best = cl;
         (void)cudaGetLastError();
     }
     return best;
@@ -1114,7 +1081,7 @@ static int af_cluster_setup()
 template <int M>
 static cudaError_t af_cluster_launch(const FEArgs& a, cudaStream_t st)
 {
-    using A = AfEngine<M>;
+    using A = AFC<M>;
     const int mx = af_cluster_setup<M>();
     if (mx < 0) return (cudaError_t)(-mx);
     const int cl = a.af_cluster;
@@ -1132,8 +1099,8 @@ static cudaError_t af_cluster_launch(const FEArgs& a, cudaStream_t st)
     cfg.stream = st;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol};
-    cudaError_t e = cudaLaunchKernelEx(&cfg, A::kernel(), fr, a.iters, a.tol, a.tw);
+    AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol, a.bar + 3};
+    cudaError_t e = cudaLaunchKernelEx(&cfg, k_af_cluster<M>, fr, a.iters, a.tol, a.tw);
     if (e == cudaSuccess) ISAR_COUNT(1);
     return e;
 }

@@ -404,15 +404,6 @@ __device__ __forceinline__ int row_out_index(int lt, int slot)
     }
 }
 
-// ---------------------------------------------------------------------------
-// Warp-level 1024-point FFT (forward, unnormalised).  Lane l holds element
-// l + 32 r in register r (r = 0..31), before and after the transform.
-// Four-step: a 32-point DFT over the registers, the twiddles W_1024^(l k),
-// a transpose of the warp's 32 x 32 block through a shared tile (row stride
-// 33, __syncwarp only), and a second 32-point DFT over the registers.  No
-// block barrier, so the warps of a CTA run their transforms independently.
-// ---------------------------------------------------------------------------
-
 // In-register 32-point forward DFT, natural order in and out:
 // X[k] = E[k] + W32^k O[k], X[k + 16] = E[k] - W32^k O[k] with E, O the
 // 16-point DFTs of the even and odd elements.
@@ -438,27 +429,6 @@ __device__ __forceinline__ void dft32_reg(float2* a)
         const float2 t = make_float2(o[k].x * c[k] + o[k].y * s[k], o[k].y * c[k] - o[k].x * s[k]);
         a[k] = cadd(e[k], t);
         a[k + 16] = csub(e[k], t);
-    }
-}
-
-// TWL: W_1024^(l k) at TWL[32 k + l] (l, k < 32) in shared memory, read
-// lane-contiguous (conflict-free); tile: this warp's 32 x 33 float2.
-// v[k] holds x[lane + 32 k] on entry and X[lane + 32 k] on return.
-__device__ __forceinline__ void warp_fft1024(float2* v, int lane, float2* tile, const float2* TWL)
-{
-    // two 32-point DFT steps sharing one copy of the code
-#pragma unroll 1
-    for (int step = 0; step < 2; ++step) {
-        dft32_reg(v);
-        if (step == 1) break;
-#pragma unroll
-        for (int k = 1; k < 32; ++k) v[k] = cmul(v[k], TWL[32 * k + lane]);
-#pragma unroll
-        for (int k = 0; k < 32; ++k) tile[lane * 33 + k] = v[k];
-        __syncwarp();
-#pragma unroll
-        for (int n = 0; n < 32; ++n) v[n] = tile[n * 33 + lane];
-        __syncwarp();
     }
 }
 

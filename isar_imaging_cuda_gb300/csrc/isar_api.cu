@@ -170,7 +170,8 @@ struct isar_ctx {
     float2* d_pc_spec = nullptr;
     size_t pc_spec_len = 0;
     unsigned* d_bar = nullptr;     // [0] autofocus grid-barrier counter, [1] its timeout flag,
-                                   // [2] range-alignment row-copy timeout flag
+                                   // [2] range-alignment row-copy timeout flag, [3] the
+                                   // cluster autofocus engine's message timeout flag
     // MTRC / post
     float2* d_st = nullptr;
     float2* d_st2 = nullptr;
@@ -540,18 +541,19 @@ int check_ctx(isar_ctx* c)
 }
 
 // Waits for the context stream and reports device-side failures: the
-// autofocus kernel's grid barrier and the range-alignment row copies set a
-// flag instead of waiting forever.
+// autofocus kernels' grid barrier and cluster messages and the range-alignment
+// row copies set a flag instead of waiting forever.
 int sync_status(isar_ctx* c)
 {
     CU(cudaStreamSynchronize(c->st));
-    unsigned flag[3] = {0, 0, 0};
+    unsigned flag[4] = {0, 0, 0, 0};
     CU(cudaMemcpy(flag, c->d_bar, sizeof(flag), cudaMemcpyDeviceToHost));
-    if (flag[1] || flag[2]) {
-        CU(cudaMemsetAsync(c->d_bar, 0, 3 * sizeof(unsigned), c->st));
+    if (flag[1] || flag[2] || flag[3]) {
+        CU(cudaMemsetAsync(c->d_bar, 0, 4 * sizeof(unsigned), c->st));
         CU(cudaStreamSynchronize(c->st));
-        return fail(ISAR_ECUDA, flag[1] ? "autofocus grid barrier timed out (image of this frame is invalid)"
-                                        : "range-alignment row copy timed out (image of this frame is invalid)");
+        return fail(ISAR_ECUDA, flag[1]   ? "autofocus grid barrier timed out (image of this frame is invalid)"
+                                : flag[2] ? "range-alignment row copy timed out (image of this frame is invalid)"
+                                          : "autofocus cluster exchange timed out (image of this frame is invalid)");
     }
     return ISAR_OK;
 }

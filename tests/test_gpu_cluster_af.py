@@ -66,6 +66,31 @@ def test_cluster_many_bins_reload_path(torch_cuda, gb300):
     assert rel_l2(got, want) < TOL_IMG
 
 
+# Bins per CTA from none (U = 2 on 16 CTAs: most CTAs only take part in the
+# exchange; half a warp owns a bin alone at 128 pulses) to more than the
+# rounds kept in shared memory (U = 256 on 4 CTAs), at every transform split.  One
+# update at U = 2: two bins of random phase are ill conditioned, further
+# updates amplify any FP32 rounding.
+@pytest.mark.parametrize("bright,U,iters", [(3, 2, 1), (9, 8, 8), (280, 256, 8)])
+@pytest.mark.parametrize("M,cl", [(128, 4), (128, 16), (256, 4), (256, 16), (512, 4), (512, 8), (1024, 8), (1024, 16)])
+def test_cluster_few_and_many_bins(torch_cuda, gb300, M, cl, bright, U, iters):
+    torch = torch_cuda
+    rng = np.random.default_rng(M + bright)
+    cut = (rng.standard_normal((M, 512)) + 1j * rng.standard_normal((M, 512))).astype(np.complex64) * 100
+    cut[:, 100:100 + bright] = (6000 * np.exp(2j * np.pi * rng.random((M, bright)))).astype(np.complex64)
+    want, tw = oracle.fast_entropy(cut, iters=iters)
+    assert tw["unit2_num"] == U
+    with ctx_for(gb300, torch, M, 2048) as ctx:
+        _cluster_or_skip(ctx, cl)
+        ctx.set_tuning(af_cluster=cl)
+        dc = to_dev(torch, cut)
+        ctx.stage_fast_entropy(dc, iters)
+        got = from_dev(torch, dc).reshape(M, 512)
+        tr = ctx.trace()
+    assert tr["unit2_num"] == U
+    assert rel_l2(got, want) < TOL_IMG
+
+
 def test_cluster_stop_criterion_equals_oracle_at_same_count(torch_cuda, gb300):
     torch = torch_cuda
     M, N = 256, 1024
