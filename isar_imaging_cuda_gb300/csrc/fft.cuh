@@ -59,8 +59,12 @@ __device__ __forceinline__ float2 twc_mul(float2 d, int j, int R)
 }
 
 // In-register DFT of length R (2..16): radix-2 decimation in frequency, then
-// the bit-reversal permutation (register renaming after unrolling).
-template <int R, bool INV>
+// the bit-reversal permutation (register renaming after unrolling).  Sums and
+// differences are packed pairs.  SRC: the inputs come from a caller's functor
+// and may be products; the first stage then stays scalar, where the compiler
+// fuses such a product into the sum (one rounding less), as the envelopes of
+// the range alignment have always been rounded.
+template <int R, bool INV, bool SRC = false>
 __device__ __forceinline__ void dft_reg(float2* a)
 {
 #pragma unroll
@@ -71,8 +75,13 @@ __device__ __forceinline__ void dft_reg(float2* a)
 #pragma unroll
             for (int k = 0; k < half; ++k) {
                 float2 u = a[s + k], v = a[s + k + half];
-                a[s + k] = cadd(u, v);
-                a[s + k + half] = twc_mul<INV>(csub(u, v), k * (R / len), R);
+                if (SRC && len == R) {
+                    a[s + k] = make_float2(u.x + v.x, u.y + v.y);
+                    a[s + k + half] = twc_mul<INV>(make_float2(u.x - v.x, u.y - v.y), k * (R / len), R);
+                } else {
+                    a[s + k] = cadd(u, v);
+                    a[s + k + half] = twc_mul<INV>(csub(u, v), k * (R / len), R);
+                }
             }
         }
     }
@@ -201,7 +210,7 @@ __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt,
                     v[b * R + r] = cmul(v[b * R + r], w);
                 }
             }
-            dft_reg<R, INV>(&v[b * R]);
+            dft_reg<R, INV, FIRST>(&v[b * R]);
             const int base = (j / NS) * NS * R + k;
             const int pb = fpad(base);
 #pragma unroll
@@ -305,7 +314,7 @@ __device__ __forceinline__ void fft8192(Src& src, Dst& dst, float2* sm, int lt, 
     for (int r = 0; r < 16; ++r) v[r] = src(lt + 512 * r);
     __syncthreads();   // the previous transform's warps are done with the scratch
     hook();
-    dft_reg<16, INV>(v);
+    dft_reg<16, INV, true>(v);
     {
         // W_8192^(lt k0): look up k0 = 1, 2, 4, 8, form the others as products
         float2 t[16];
