@@ -104,7 +104,9 @@ typedef struct {
     int ra_rows_per_cta;      /* rows per CTA of the envelope accumulation (4)        */
     int ra_rows_final;        /* rows per CTA of the final range transform (4)        */
     int af_cluster;           /* autofocus engine: 0 = one cooperative grid of 128    */
-                              /* CTAs; 4, 8, 16 = one thread-block cluster per frame  */
+                              /* CTAs (up to 512 pulses a cluster of 16 where one can */
+                              /* be launched: same results, no stop criterion);       */
+                              /* 4, 8, 16 = one thread-block cluster per frame        */
     float af_tol;             /* stop once the entropy of the selected bins changes   */
                               /* by <= af_tol * |entropy| per iteration (mean over 4, */
                               /* checked every 4th iteration; cluster engine; 0 = off)*/

@@ -358,13 +358,15 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, i
 // q = conj(g) .* h and writes its partial row sums to P[m][b].  After a grid
 // barrier CTA b sums the rows m = b, b+G, ... over all partials and writes
 // phase[m] = sigma / |sigma|; a second barrier publishes the new phase.
-// phase: in the Doppler-tracking start, out the final phase.
+// phase: in the Doppler-tracking start, out the final phase.  Frames with
+// fewer than min_u bins are left alone.
 template <int M>
 __global__ void __launch_bounds__(4 * (M / 16))
 k_af_persist(const float2* __restrict__ cut, const int* __restrict__ bins, const int* __restrict__ fdec,
              float2* phase, float2* P, unsigned* bar, int* err, int iters, const float2* __restrict__ tw,
-             BarrierTest bt)
+             BarrierTest bt, int min_u)
 {
+    if (fdec[1] < min_u) return;   // the whole grid, before any barrier
     using F = FFTShape<M>;
     constexpr int TEAMS = 4;
     extern __shared__ float4 dyn_smem[];
@@ -467,13 +469,14 @@ k_af_persist(const float2* __restrict__ cut, const int* __restrict__ bins, const
 // and drives the optional stop criterion (iterations that need it take a
 // cluster barrier more).
 //
-// Bound by latency: at 8 bins per CTA and 256 pulses an iteration is ~2700
-// clocks of transforms and ~2000 of reduction and messages.  Per iteration
-// (U = 64; team transforms with block barriers, gathers by remote loads and
-// two cluster barriers before -> now): 128 pulses 5.4 -> 2.1 us (4 CTAs),
-// 256 pulses 6.2 -> 2.3 (8 CTAs), 512 pulses 8.1 -> 3.4 (16 CTAs), 1024 pulses
-// 6.1 -> 5.2 (16 CTAs).  Two warps per bin (16 elements per lane, two tile
-// exchanges) measured 5.8 us at 1024 and 3.8 us at 512 pulses.
+// Bound by latency: at 4 bins per CTA and 256 pulses an iteration is ~1700
+// clocks of transforms, 500 of the two reductions and 500 for each message.
+// Per iteration at U = 64 / 128 (team transforms with block barriers, gathers
+// by remote loads and two cluster barriers before -> now): 128 pulses
+// 5.4 / 6.2 -> 1.9 / 2.9 us (4 CTAs), 256 pulses 6.2 / 6.4 -> 1.9 / 3.0
+// (8 CTAs), 512 pulses 8.1 / 8.8 -> 2.8 / 3.6 (16 CTAs), 1024 pulses
+// 6.1 / 7.5 -> 4.2 / 5.9 (16 CTAs).  Two warps per bin (16 elements per lane,
+// two tile exchanges) measured slower at 512 and 1024 pulses.
 // ---------------------------------------------------------------------------
 template <int M>
 struct AFC {
@@ -484,11 +487,11 @@ struct AFC {
     static constexpr int WARPS = 8;
     static constexpr int THREADS = WARPS * 32;
     static constexpr int BINS = WARPS * BW;                        // bins per round
-    static constexpr int CTAS = M >= 512 ? 1 : 2;                  // per SM (registers)
+    static constexpr int CTAS = M >= 1024 ? 1 : 2;                 // per SM (registers)
     static constexpr int S1 = L + Q;   // tile row stride: both directions free of bank conflicts
     static constexpr int TILE = P * S1;                            // per bin; also its M partial sums
     static constexpr int NSLOT = 2;                                // cached rounds
-    static constexpr int BUF = M + 256;                            // [CL][M / CL + pad]
+    static constexpr int BUF = M + 64;                             // [CL][M / CL + pad]
     static constexpr size_t SMEM_F2 =
         (size_t)M + BUF + (size_t)BINS * TILE + (size_t)NSLOT * BINS * M + (size_t)M + (size_t)P * Q;
     static constexpr size_t SMEM = SMEM_F2 * sizeof(float2) + 64 * sizeof(double);
@@ -511,6 +514,7 @@ struct AFFrame {
                            // out (warm start), or null
     float2* gcol;          // [U][M] scratch: contiguous copy of the bin columns
     unsigned* err;         // set when a message between the CTAs does not arrive
+    int max_u;             // the kernel leaves frames with more bins alone
 };
 
 // The DFT over q (q = lane mod Q) of the elements c = 0..P-1 that Q
@@ -648,6 +652,17 @@ __device__ __forceinline__ float2 times_abs(float2 v, bool ent, float& s1, float
     return make_float2(v.x * a, v.y * a);
 }
 
+// s / |s| with one reciprocal square root and a Newton step (as exact as the
+// square root and two divisions it stands for, a third of their latency).
+// As s / sqrtf(|s|^2): 0 / 0 is NaN, an overflowing |s|^2 gives 0.
+__device__ __forceinline__ float2 unit(float2 s)
+{
+    const float p = s.x * s.x + s.y * s.y;
+    float y = rsqrtf(p);
+    if (p > 0.0f && p < CUDART_INF_F) y = fmaf(y, fmaf(-0.5f * p * y, y, 0.5f), y);
+    return make_float2(s.x * y, s.y * y);
+}
+
 // With a learned start (AFFrame::alt) the engine runs two legs: the
 // autofocus from the learned start until the stop criterion (`tol`), then the
 // plain autofocus, the reference's algorithm (Doppler-tracking start, `iters`
@@ -662,7 +677,7 @@ __device__ __forceinline__ float2 times_abs(float2 v, bool ent, float& s1, float
 // ([U][M], written by the loading lanes themselves on entry), and successive
 // sweeps alternate direction so that the NSLOT rounds left in shared memory
 // by one sweep are the first of the next.
-template <int M>
+template <int M, int CL>
 __global__ void __launch_bounds__(AFC<M>::THREADS, AFC<M>::CTAS)
 k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
 {
@@ -670,7 +685,6 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     using A = AFC<M>;
     constexpr int P = A::P, L = A::L, Q = A::Q;
     cg::cluster_group cl = cg::this_cluster();
-    const int CL = (int)cl.num_blocks();
     const int r = (int)cl.block_rank();
     extern __shared__ float4 dyn_smem[];
     __shared__ __align__(8) uint64_t bar_part, bar_ph;          // partial sums, phase slices arrived
@@ -695,6 +709,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     for (int i = tid; i < P * Q; i += A::THREADS) T2[i] = tw[(i / Q) * (i & (Q - 1)) * (kTwN / L)];
     float2* ta = tiles + slot * A::TILE;
     const int U = f.fdec[1];
+    if (U > f.max_u) return;   // the whole cluster, before any message
     const int bpc = (U + CL - 1) / CL;
     const int b0 = r * bpc;
     const int nb = max(0, min(bpc, U - b0));
@@ -706,9 +721,14 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     for (int m = tid; m < M; m += A::THREADS) ph[m] = f.phase[m];
     for (int j = 0; j < nrd; ++j) {
         const int t = j * A::BINS + slot;
-        if (t >= nb || (j >= A::NSLOT && !reload)) continue;
-        const int b = f.bins[b0 + t];
+        if (j >= A::NSLOT && !reload) continue;
         float2* g = cache + ((size_t)(j % A::NSLOT) * A::BINS + slot) * M;
+        if (t >= nb) {   // a half-empty warp computes on zeros
+            if (A::BW == 2 && j < A::NSLOT)
+                for (int i = 0; i < P; ++i) g[l + L * i] = make_float2(0.0f, 0.0f);
+            continue;
+        }
+        const int b = f.bins[b0 + t];
         float2* gg = gw + (size_t)j * A::BINS * M;
 #pragma unroll 4
         for (int i = 0; i < P; ++i) {
@@ -721,12 +741,12 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     cl.sync();   // every CTA of the cluster runs and has its mbarriers: messages may be sent
 
     const float invM = 1.0f / (float)M;
-    const int rows = M / CL;
-    const int lg_rows = 31 - __clz(rows);
+    constexpr int rows = M / CL;
     // threads per row of the cluster reduction, and the row stride of buf that
     // keeps their reads in different banks
-    const int tpr = min(CL, A::THREADS / rows);
-    const int bs = rows + 16 / tpr + ((16 / tpr) & 1);
+    constexpr int tpr = CL < A::THREADS / rows ? CL : A::THREADS / rows;
+    constexpr int bs = rows + 16 / tpr + ((16 / tpr) & 1);
+    static_assert(CL * bs <= A::BUF && rows * tpr <= A::THREADS && (rows * tpr) % 32 == 0, "cluster reduction");
     // twiddles of the short transforms in registers
     constexpr bool kRegTw = P <= 8;
     float2 w1[kRegTw ? P : 1], w2[kRegTw ? P : 1];
@@ -760,20 +780,19 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
         for (int jj = 0; jj < nrd; ++jj) {
             const int j = back ? nrd - 1 - jj : jj;
             if (j * A::BINS + warp * A::BW >= nb) continue;   // warp-uniform; no block barrier inside
-            const bool valid = A::BW == 1 || j * A::BINS + slot < nb;
             float2* g = cache + ((size_t)(j % A::NSLOT) * A::BINS + slot) * M;
             __syncwarp();   // the slot and the tile of the previous round are read
-            if (jj >= A::NSLOT && valid) {   // only when reload: read the copy in gcol
+            if (jj >= A::NSLOT) {   // only when reload: read the copy in gcol
+                const bool valid = A::BW == 1 || j * A::BINS + slot < nb;
                 const float4* src = reinterpret_cast<const float4*>(gw + (size_t)j * A::BINS * M);
                 float4* dst = reinterpret_cast<float4*>(g);
 #pragma unroll 4
-                for (int i = l; i < M / 2; i += L) dst[i] = src[i];
+                for (int i = l; i < M / 2; i += L) dst[i] = valid ? src[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
             __syncwarp();
             float2 v[P];
 #pragma unroll
-            for (int i = 0; i < P; ++i)
-                v[i] = valid ? cmul(ph[l + L * i], g[l + L * i]) : make_float2(0.0f, 0.0f);
+            for (int i = 0; i < P; ++i) v[i] = cmul(ph[l + L * i], g[l + L * i]);
             if constexpr (Q == 1) {
                 // pass 0: T = FFT(phase * g); pass 1: conj(IFFT(T |T|)) * M as
                 // the forward FFT of conj(T |T|)
@@ -834,13 +853,11 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
 #pragma unroll
                 for (int k = 1; k < P; ++k) v[k] = cmulc(t1(k), v[k]);
                 dft_reg<P, true>(v);
-                if (valid) {
 #pragma unroll
-                    for (int i = 0; i < P; ++i) {
-                        const float2 x = g[l + L * i];   // conj(x) v
-                        pacc[i].x = fmaf(x.x, v[i].x, fmaf(x.y, v[i].y, pacc[i].x));
-                        pacc[i].y = fmaf(x.x, v[i].y, fmaf(-x.y, v[i].x, pacc[i].y));
-                    }
+                for (int i = 0; i < P; ++i) {
+                    const float2 x = g[l + L * i];   // conj(x) v
+                    pacc[i].x = fmaf(x.x, v[i].x, fmaf(x.y, v[i].y, pacc[i].x));
+                    pacc[i].y = fmaf(x.x, v[i].y, fmaf(-x.y, v[i].x, pacc[i].y));
                 }
             }
         }
@@ -861,7 +878,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
                     a = cadd(a, make_float2(t.x, t.y));
                     b = cadd(b, make_float2(t.z, t.w));
                 }
-            const int to = m >> lg_rows;
+            const int to = m / rows;
             msg_send2(cluster_addr(smem_u32(&buf[r * bs + (m & (rows - 1))]), to), cluster_addr(smem_u32(&bar_part), to),
                       a, b);
         }
@@ -947,18 +964,23 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
             }
             // tpr neighbouring threads add a row's CL partial sums (fixed
             // tree) and send its new phase to CL / tpr CTAs each
-            for (int idx = tid; idx < rows * tpr; idx += A::THREADS) {
-                const int part = idx & (tpr - 1), ml = idx / tpr;
+            if (tid < rows * tpr) {
+                const int part = tid & (tpr - 1), ml = tid / tpr;
                 float2 s = buf[part * bs + ml];
-                for (int x = part + tpr; x < CL; x += tpr) s = cadd(s, buf[x * bs + ml]);
+#pragma unroll
+                for (int x = tpr; x < CL; x += tpr) s = cadd(s, buf[(part + x) * bs + ml]);
+#pragma unroll
                 for (int o = tpr >> 1; o > 0; o >>= 1) {
-                    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-                    s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+                    float2 t;
+                    t.x = __shfl_xor_sync(0xffffffffu, s.x, o);
+                    t.y = __shfl_xor_sync(0xffffffffu, s.y, o);
+                    s = cadd(s, t);
                 }
-                const float a = sqrtf(s.x * s.x + s.y * s.y);
-                s = make_float2(s.x / a, s.y / a);
-                for (int to = part; to < CL; to += tpr)
-                    msg_send(cluster_addr(smem_u32(&ph[r * rows + ml]), to), cluster_addr(smem_u32(&bar_ph), to), s);
+                s = unit(s);
+#pragma unroll
+                for (int x = 0; x < CL; x += tpr)
+                    msg_send(cluster_addr(smem_u32(&ph[r * rows + ml]), part + x),
+                             cluster_addr(smem_u32(&bar_ph), part + x), s);
             }
             if (tid == 0) msg_expect(&bar_ph, M * sizeof(float2));
             msg_wait(&bar_ph, par >> 1, &dead, f.err);
@@ -1038,34 +1060,49 @@ __global__ void k_af_apply2(float2* __restrict__ cut, const float2* __restrict__
 template <int M>
 static constexpr int af_cb() { return M >= 512 ? 8 : (M >= 256 ? 16 : 32); }
 
+using AfKernel = void (*)(AFFrame, int, float, const float2*);
+template <int M>
+static AfKernel af_kernel(int cl)
+{
+    return cl == 16 ? k_af_cluster<M, 16> : cl == 8 ? k_af_cluster<M, 8> : k_af_cluster<M, 4>;
+}
+
+// The launch of one cluster of cl CTAs (`at` must outlive the configuration).
+template <int M>
+static cudaLaunchConfig_t af_cluster_config(int cl, cudaStream_t st, cudaLaunchAttribute* at)
+{
+    cudaLaunchConfig_t cfg = {};
+    at->id = cudaLaunchAttributeClusterDimension;
+    at->val.clusterDim.x = cl;
+    at->val.clusterDim.y = 1;
+    at->val.clusterDim.z = 1;
+    cfg.gridDim = dim3(cl);
+    cfg.blockDim = dim3(AFC<M>::THREADS);
+    cfg.dynamicSmemBytes = AFC<M>::SMEM;
+    cfg.stream = st;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
 // Cluster engine set-up (once per device): shared-memory limit, non-portable
 // cluster sizes, and the largest of 16/8/4 CTAs per cluster that can be
 // resident.  Returns that size, 0 if none, or a negative cudaError_t.
 template <int M>
 static int af_cluster_probe()
 {
-    using A = AFC<M>;
-    cudaError_t e;
-    if ((e = cudaFuncSetAttribute(k_af_cluster<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)A::SMEM)))
-        return -(int)e;
-    if ((e = cudaFuncSetAttribute(k_af_cluster<M>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))) {
-        (void)cudaGetLastError();
-    }
     int best = 0;
-    for (int cl = 16; cl >= 4 && best == 0; cl >>= 1) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = cl;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.gridDim = dim3(cl);
-        cfg.blockDim = dim3(A::THREADS);
-        cfg.dynamicSmemBytes = A::SMEM;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
+    for (int cl : {16, 8, 4}) {
+        const AfKernel k = af_kernel<M>(cl);
+        cudaError_t e;
+        if ((e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AFC<M>::SMEM)))
+            return -(int)e;
+        if (cl > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
+            (void)cudaGetLastError();
+        cudaLaunchAttribute at;
+        const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, nullptr, &at);
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, k_af_cluster<M>, &cfg) == cudaSuccess && n > 0) best = cl;
+        if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0 && best == 0) best = cl;
         (void)cudaGetLastError();
     }
     return best;
@@ -1079,28 +1116,16 @@ static int af_cluster_setup()
 }
 
 template <int M>
-static cudaError_t af_cluster_launch(const FEArgs& a, cudaStream_t st)
+static cudaError_t af_cluster_launch(const FEArgs& a, int cl, int max_u, cudaStream_t st)
 {
-    using A = AFC<M>;
     const int mx = af_cluster_setup<M>();
     if (mx < 0) return (cudaError_t)(-mx);
-    const int cl = a.af_cluster;
     if (cl != 4 && cl != 8 && cl != 16) return cudaErrorInvalidValue;
     if (cl > mx) return cudaErrorInvalidClusterSize;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = cl;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3(cl);
-    cfg.blockDim = dim3(A::THREADS);
-    cfg.dynamicSmemBytes = A::SMEM;
-    cfg.stream = st;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol, a.bar + 3};
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_af_cluster<M>, fr, a.iters, a.tol, a.tw);
+    cudaLaunchAttribute at;
+    const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, st, &at);
+    AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol, a.bar + 3, max_u};
+    cudaError_t e = cudaLaunchKernelEx(&cfg, af_kernel<M>(cl), fr, a.iters, a.tol, a.tw);
     if (e == cudaSuccess) ISAR_COUNT(1);
     return e;
 }
@@ -1169,12 +1194,27 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
         if ((e = nn::forward(*a.ws_w, *a.ws_a, 1, M, a.ws_err, st))) return e;
         if ((e = nn::ws_phase(a.ws_psi, a.ws_a->out, M, a.ws_phase, st))) return e;
     }
-    if (a.iters > 0 && a.af_cluster > 0) {
-        cudaError_t e = af_cluster_launch<M>(a, st);
+    // Engine 0 up to 512 pulses runs as one 16-CTA cluster where one can be
+    // launched: per iteration, cooperative grid -> cluster, U = 64 and 256:
+    // 6.4 -> 1.6 and 6.5 -> 2.1 us at 128 pulses, 6.5 -> 1.6 and 6.5 -> 3.1 at 256,
+    // 7.6 -> 2.8 and 7.8 -> 6.0 at 512.  Only at 512 pulses and the largest U,
+    // 512 (profiles below one count: the integer mean of the threshold is 0), is
+    // the grid ahead (8 against 10 us): both kernels are launched there and the
+    // one that the frame's U does not select returns at once.  At 1024 pulses
+    // the grid is ahead from U = 256 (9.0 against 9.9; 8.2 against 4.2 at U = 64)
+    // and engine 0 stays the grid, as it does under the barrier's test hook.
+    const bool auto16 =
+        a.af_cluster == 0 && M <= 512 && !a.bar_test.active() && af_cluster_setup<M>() >= 16;
+    const int cl = auto16 ? 16 : a.af_cluster;
+    const int max_u = auto16 && M == 512 ? 256 : C;
+    if (a.iters > 0 && cl > 0) {
+        cudaError_t e = af_cluster_launch<M>(a, cl, max_u, st);
         if (e) return e;
-    } else if (a.iters > 0) {
+    }
+    if (a.iters > 0 && (cl == 0 || max_u < C)) {
         cudaError_t e;
         if ((e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), st))) return e;
+        int min_u = cl == 0 ? 0 : max_u + 1;
         const float2* cut = a.cut;
         const int* bins = a.bins;
         const int* fdec = a.fdec;
@@ -1186,7 +1226,7 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
         const float2* tw = a.tw;
         BarrierTest bt = a.bar_test;
         void* args[] = {(void*)&cut, (void*)&bins, (void*)&fdec, (void*)&phase, (void*)&P,
-                        (void*)&bar, (void*)&err, (void*)&iters, (void*)&tw, (void*)&bt};
+                        (void*)&bar, (void*)&err, (void*)&iters, (void*)&tw, (void*)&bt, (void*)&min_u};
         if ((e = cudaLaunchCooperativeKernel((const void*)k_af_persist<M>, dim3(grid_p), dim3(4 * F::T), args, smem_p,
                                              st)))
             return e;

@@ -90,6 +90,7 @@ constexpr unsigned long long kSpinLimit = 1ull << 22;
 struct BarrierTest {
     unsigned long long limit = kSpinLimit;
     unsigned extra = 0;
+    bool active() const { return limit != kSpinLimit || extra != 0; }
 };
 
 struct FEArgs {
@@ -108,9 +109,10 @@ struct FEArgs {
     unsigned* bar;           // [0] grid-barrier counter, [1] barrier timeout flag
     BarrierTest bar_test;    // poll limit and target offset of the grid barrier
     const float2* tw;
-    // Autofocus engine: 0 = one cooperative grid (128 CTAs, grid barriers);
-    // 4, 8 or 16 = one thread-block cluster of that many CTAs per frame
-    // (distributed shared memory, no grid barrier).
+    // Autofocus engine: 4, 8 or 16 = one thread-block cluster of that many
+    // CTAs per frame (distributed shared memory, no grid barrier); 0 = one
+    // cooperative grid (128 CTAs, grid barriers) or, up to 512 pulses, a
+    // cluster of 16 where one can be launched, without a stop criterion.
     int af_cluster;
     // Entropy stop criterion (cluster engine): stop once the entropy of the
     // selected bins changes by <= tol * |entropy| per iteration (mean over

@@ -91,6 +91,30 @@ def test_cluster_few_and_many_bins(torch_cuda, gb300, M, cl, bright, U, iters):
     assert rel_l2(got, want) < TOL_IMG
 
 
+# Engine 0 picks its kernel by the pulse count and, at 512 pulses, by U on the
+# device: 256 bins on the cluster, 512 (profiles below one count, whose
+# integer mean is 0) on the cooperative grid.  Both give the oracle's result
+# and leave the trace's engine fields as engine 0 reports them.
+@pytest.mark.parametrize("M", [128, 256, 512, 1024])
+@pytest.mark.parametrize("bright,scale,U", [(40, 6000.0, 32), (280, 6000.0, 256), (512, 0.5, 512)])
+def test_engine0_every_bin_count(torch_cuda, gb300, M, bright, scale, U):
+    torch = torch_cuda
+    rng = np.random.default_rng(3 * M + bright)
+    cut = (rng.standard_normal((M, 512)) + 1j * rng.standard_normal((M, 512))).astype(np.complex64) * scale / 60
+    k = (512 - bright) // 2
+    cut[:, k:k + bright] = (scale * np.exp(2j * np.pi * rng.random((M, bright)))).astype(np.complex64)
+    want, tw = oracle.fast_entropy(cut, iters=6)
+    assert tw["unit2_num"] == U
+    with ctx_for(gb300, torch, M, 2048) as ctx:
+        ctx.set_tuning(af_cluster=0)
+        dc = to_dev(torch, cut)
+        ctx.stage_fast_entropy(dc, 6)
+        got = from_dev(torch, dc).reshape(M, 512)
+        tr = ctx.trace()
+    assert tr["unit2_num"] == U and np.isnan(tr["af_entropy"])
+    assert rel_l2(got, want) < TOL_IMG
+
+
 def test_cluster_stop_criterion_equals_oracle_at_same_count(torch_cuda, gb300):
     torch = torch_cuda
     M, N = 256, 1024
