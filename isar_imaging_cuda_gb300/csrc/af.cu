@@ -38,6 +38,7 @@ k_fe_stats(const float2* __restrict__ cut, int M, int rows_max, int R, float* __
         const int r1 = min(r0 + R, rows_max);
         for (int c = tid; c < C; c += blockDim.x) {
             float mx = 0.0f;
+#pragma unroll 8
             for (int r = r0; r < r1; ++r) {
                 const float2 v = cut[(size_t)r * C + c];
                 mx = fmaxf(mx, sqrtf(v.x * v.x + v.y * v.y));
@@ -48,6 +49,7 @@ k_fe_stats(const float2* __restrict__ cut, int M, int rows_max, int R, float* __
     const int w = tid >> 5, lane = tid & 31;
     for (int m = r0 + w; m < min(r0 + R, M - 1); m += blockDim.x >> 5) {
         float2 s = make_float2(0.0f, 0.0f);
+#pragma unroll
         for (int c = lane; c < C; c += 32) {
             const float2 a = cut[(size_t)m * C + c];
             const float2 b = cut[(size_t)(m + 1) * C + c];
@@ -88,77 +90,97 @@ k_af_doppler(const float2* __restrict__ cut, const int* __restrict__ bins, const
     if (lane == 0) dsum[m] = s;
 }
 
-// One CTA (1024 threads).  Optional target count (phase_adjustment.cu:180-194):
-// colmax, mean with an int accumulator (Q3), threshold 1.48*mean.  Then the
 // Doppler phase: psi = arg(s), Phi = inclusive scan, phase[0] = 0,
-// phase[m+1] = exp(-j*Phi[m]) (phase_adjustment.cu:17-31).
+// phase[m+1] = exp(-j*Phi[m]) (phase_adjustment.cu:17-31); M threads per CTA,
+// warp b of CTA b writes the phases of its 32 pulses.  Every CTA scans all of psi:
+// in 64-bit fixed point (units of 2^-50 rad, exact for the float angles down
+// to 2^-27 rad), which is faster than adding doubles and as exact.  The
+// double sine and cosine are what the kernel is bound by (FP64 issues ~2 per
+// clock and SM): spread over M / 32 CTAs, one warp each (one CTA took
+// 25000 clocks at 1024 pulses, 8900 of them in a scan of doubles).
+// CTA 0 also counts the targets (phase_adjustment.cu:180-194) when nparts > 0:
+// colmax, mean with an int accumulator (Q3), threshold 1.48*mean.
 // fdec: [0] tgt_num, [1] U.
 __global__ void __launch_bounds__(1024)
 k_fe_phase(const float* __restrict__ cmax_part, int nparts, const float2* __restrict__ dsum, int M,
            float2* __restrict__ phase, int* __restrict__ fdec)
 {
-    __shared__ double sc[1024];
+    __shared__ long long s_tot[32];
+    __shared__ unsigned s_nan[32];
     __shared__ int s_cnt[32];
-    __shared__ long long s_sum[32];
+    __shared__ int s_sum[32];
     const int tid = threadIdx.x;
-    const int lane = tid & 31, w = tid >> 5;
-    if (nparts > 0) {
-        float mx = 0.0f;
-        int iv = 0;
-        if (tid < C) {
-            for (int p = 0; p < nparts; ++p) mx = fmaxf(mx, cmax_part[(size_t)p * C + tid]);
-            iv = (int)mx;
-        }
-        long long sum = iv;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-        if (lane == 0) s_sum[w] = sum;
-        __syncthreads();
-        if (tid == 0) {
-            long long t = 0;
-            for (int i = 0; i < 32; ++i) t += s_sum[i];
-            s_sum[0] = t;
-        }
-        __syncthreads();
-        const float mean_val = (float)(int)s_sum[0] / (float)C;
-        const float thr = 1.48f * mean_val;
-        int cnt = (tid < C && mx > thr) ? 1 : 0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-        if (lane == 0) s_cnt[w] = cnt;
-        __syncthreads();
-        if (tid == 0) {
-            int t = 0;
-            for (int i = 0; i < 32; ++i) t += s_cnt[i];
-            // U = nextPow2(tgt_num / 2) (common.cu:521-529)
-            int n = t / 2, u = 1;
-            while (n >> 1) {
-                u <<= 1;
-                n >>= 1;
-            }
-            fdec[0] = t;
-            fdec[1] = u << 1;
-        }
-    }
-    // inclusive scan of arg(s) in double
-    double v = 0.0;
+    const int lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
+    // inclusive scan of arg(s); a NaN reaches every later phase
+    long long v = 0;
+    bool bad = false;
     if (tid < M - 1) {
         const float2 s = dsum[tid];
-        v = (double)atan2f(s.y, s.x);
+        const float psi = atan2f(s.y, s.x);
+        bad = isnan(psi);
+        v = bad ? 0 : __float2ll_rn(psi * 1125899906842624.0f);   // 2^50, exact
     }
-    sc[tid] = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const long long t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
+    }
+    const unsigned nans = __ballot_sync(0xffffffffu, bad);
+    if (lane == 31) {
+        s_tot[w] = v;
+        s_nan[w] = nans;
+    }
     __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        double add = (tid >= o) ? sc[tid - o] : 0.0;
-        __syncthreads();
-        sc[tid] += add;
-        __syncthreads();
+    if (w == (int)blockIdx.x) {   // this CTA's 32 pulses
+        unsigned any = nans & ((2u << lane) - 1u);
+        for (int i = 0; i < w; ++i) {
+            v += s_tot[i];
+            any |= s_nan[i];
+        }
+        if (tid < M - 1) {
+            double sn, cs;
+            sincos(any ? CUDART_NAN : (double)v * 8.8817841970012523234e-16, &sn, &cs);   // 2^-50
+            phase[tid + 1] = make_float2((float)cs, (float)-sn);
+        }
+        if (tid == 0) phase[0] = make_float2(0.0f, 0.0f);
     }
-    if (tid == 0) phase[0] = make_float2(0.0f, 0.0f);
-    if (tid < M - 1) {
-        double sn, cs;
-        sincos(sc[tid], &sn, &cs);
-        phase[tid + 1] = make_float2((float)cs, (float)-sn);
+    if (nparts == 0 || blockIdx.x != 0) return;
+    float mx[C / 128];   // M >= 128 threads: up to four columns each
+    int isum = 0;
+#pragma unroll
+    for (int q = 0; q < C / 128; ++q) {
+        const int c = tid + q * (int)blockDim.x;
+        mx[q] = 0.0f;
+        if (c < C) {
+#pragma unroll 8
+            for (int p = 0; p < nparts; ++p) mx[q] = fmaxf(mx[q], cmax_part[(size_t)p * C + c]);
+            isum += (int)mx[q];
+        }
+    }
+    // the int accumulator wraps, as the reference's does
+    isum = (int)__reduce_add_sync(0xffffffffu, (unsigned)isum);
+    if (lane == 0) s_sum[w] = isum;
+    __syncthreads();
+    isum = (int)__reduce_add_sync(0xffffffffu, lane < nw ? (unsigned)s_sum[lane] : 0u);
+    const float mean_val = (float)isum / (float)C;
+    const float thr = 1.48f * mean_val;
+    int cnt = 0;
+#pragma unroll
+    for (int q = 0; q < C / 128; ++q) cnt += (tid + q * (int)blockDim.x < C && mx[q] > thr) ? 1 : 0;
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    if (lane == 0) s_cnt[w] = cnt;
+    __syncthreads();
+    if (tid == 0) {
+        int t = 0;
+        for (int i = 0; i < nw; ++i) t += s_cnt[i];
+        // U = nextPow2(tgt_num / 2) (common.cu:521-529)
+        int n = t / 2, u = 1;
+        while (n >> 1) {
+            u <<= 1;
+            n >>= 1;
+        }
+        fdec[0] = t;
+        fdec[1] = u << 1;
     }
 }
 
@@ -233,14 +255,14 @@ k_fe_colfft(const float2* __restrict__ cut, const float2* __restrict__ phase, do
     }
 }
 
-// One element per thread of a 512-thread CTA, sorted so that thread i ends
-// with the i-th element in the strict order `before`: strides below 32 are
-// exchanged by warp shuffles, larger ones through shared memory (10 of the
-// 45 stages).  `before` must be a strict order; equal elements are
-// interchangeable (they end in either of their places).
+// One element per thread of a 512-thread CTA, sorted ascending by (key, tie):
+// thread i ends with the i-th element.  Strides below 32 are exchanged by warp
+// shuffles, larger ones through shared memory (10 of the 45 stages).  Keys are
+// unsigned integers (double_order): compares of doubles run on the FP64 pipe,
+// which issues ~2 per clock and SM.
 struct SelKey {
-    double key;
-    int tie;   // tie-break (smaller first)
+    unsigned long long key;
+    int tie;   // distinct
     int val;   // payload
 };
 __device__ __forceinline__ SelKey shfl_xor_key(const SelKey& v, int j)
@@ -251,10 +273,16 @@ __device__ __forceinline__ SelKey shfl_xor_key(const SelKey& v, int j)
     w.val = __shfl_xor_sync(0xffffffffu, v.val, j);
     return w;
 }
-template <class Before>
-__device__ __forceinline__ void sort512(SelKey& v, SelKey* sm, Before before)
+// Unsigned order of a double (ascending).
+__device__ __forceinline__ unsigned long long double_order(double d)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d + 0.0);   // -0 orders as 0
+    return b ^ ((b >> 63) ? ~0ull : 1ull << 63);
+}
+__device__ __forceinline__ void sort512(SelKey& v, SelKey* sm)
 {
     const int i = threadIdx.x;
+#pragma unroll 1
     for (int k = 2; k <= C; k <<= 1)
         for (int j = k >> 1; j > 0; j >>= 1) {
             SelKey w;
@@ -266,9 +294,9 @@ __device__ __forceinline__ void sort512(SelKey& v, SelKey* sm, Before before)
             } else {
                 w = shfl_xor_key(v, j);
             }
-            const bool up = (i & k) == 0;      // this region ascends in `before` order
+            const bool up = (i & k) == 0;      // this region ascends
             const bool lower = (i & j) == 0;   // i is the lower index of its pair
-            const bool v_first = before(v, w);
+            const bool v_first = v.key < w.key || (v.key == w.key && v.tie < w.tie);
             if (!((lower == up) ? v_first : !v_first)) v = w;
         }
 }
@@ -277,44 +305,53 @@ __device__ __forceinline__ void sort512(SelKey& v, SelKey* sm, Before before)
 // column per thread: stable sort by energy (descending), keep tgt_num, stable
 // sort by entropy (ascending), keep U (indices beyond tgt_num are 0, as
 // device_vector::resize pads), sort the kept indices.  NaN keys sort last.
-// The stable sorts are strict orders with the position as tie-break.
+// The stable sorts are strict orders with the position as tie-break; the kept
+// indices are put in order by a prefix count of their columns' flags.
+// Latency of one CTA: ~19500 clocks, bound by the shuffles of its 90 stages (33 us
+// with double keys and a third sort).
 __global__ void __launch_bounds__(C)
 k_fe_select(const double* __restrict__ E, const double* __restrict__ H, int* __restrict__ fdec,
             int* __restrict__ bins)
 {
     __shared__ SelKey sm[C];
-    const int tid = threadIdx.x;
+    __shared__ int s_flag[C];
+    __shared__ int s_cnt[C / 32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int tgt = fdec[0], U = fdec[1];
     SelKey v;
+    const double h_own = H[tid];
     {
         const double e = E[tid];
-        v.key = isnan(e) ? -CUDART_INF : e;
+        v.key = ~double_order(isnan(e) ? -CUDART_INF : e);   // descending
         v.tie = tid;
         v.val = tid;
     }
-    sort512(v, sm, [](const SelKey& a, const SelKey& b) {
-        return a.key > b.key || (a.key == b.key && a.tie < b.tie);
-    });
+    sort512(v, sm);
     // second key: entropy of the first tgt entries; the rest are sentinels
+    __syncthreads();
+    double* s_h = reinterpret_cast<double*>(sm);
+    s_h[tid] = h_own;
+    s_flag[tid] = 0;
+    __syncthreads();
     {
-        double h = (tid < tgt) ? H[v.val] : CUDART_INF;
+        double h = (tid < tgt) ? s_h[v.val] : CUDART_INF;
         if (isnan(h)) h = CUDART_INF;
-        v.key = h;
+        v.key = double_order(h);
         v.tie = (tid < tgt) ? tid : (C + tid);
     }
-    sort512(v, sm, [](const SelKey& a, const SelKey& b) {
-        return a.key < b.key || (a.key == b.key && a.tie < b.tie);
-    });
-    // keep U, pad with 0, sort ascending
-    {
-        int b = 0x7fffffff;
-        if (tid < U) b = (tid < tgt) ? v.val : 0;
-        v.key = 0.0;
-        v.tie = 0;
-        v.val = b;
-    }
-    sort512(v, sm, [](const SelKey& a, const SelKey& b) { return a.val < b.val; });
-    if (tid < U) bins[tid] = v.val;
+    __syncthreads();
+    sort512(v, sm);
+    // the first U of the tgt kept entries; U > tgt pads with index 0 in front
+    const int kept = min(U, tgt), pad = U - kept;
+    if (tid < kept) s_flag[v.val] = 1;
+    __syncthreads();
+    const unsigned b = __ballot_sync(0xffffffffu, s_flag[tid] != 0);
+    if (lane == 0) s_cnt[w] = __popc(b);
+    __syncthreads();
+    int before = 0;
+    for (int i = 0; i < w; ++i) before += s_cnt[i];
+    if (s_flag[tid]) bins[pad + before + __popc(b & ((1u << lane) - 1u))] = tid;
+    if (tid < pad) bins[tid] = 0;
 }
 
 // Grid-wide barrier for cooperative launches (all CTAs co-resident): arrive
@@ -1175,7 +1212,7 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
     const int nparts = (rows_max + R - 1) / R;
     k_fe_stats<<<(M + R - 1) / R, 256, 0, st>>>(a.cut, M, rows_max, R, a.cmax_part, a.dsum);
     ISAR_COUNT(1);
-    k_fe_phase<<<1, 1024, 0, st>>>(a.cmax_part, nparts, a.dsum, M, a.phase, a.fdec);
+    k_fe_phase<<<M / 32, M, 0, st>>>(a.cmax_part, nparts, a.dsum, M, a.phase, a.fdec);
     ISAR_COUNT(1);
     k_fe_colfft<M, CB><<<C / CB, CB * F::T, smem, st>>>(a.cut, a.phase, a.E, a.H, a.tw);
     ISAR_COUNT(1);
@@ -1183,7 +1220,7 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
     ISAR_COUNT(1);
     k_af_doppler<<<(M * 32 + 255) / 256, 256, 0, st>>>(a.cut, a.bins, a.fdec, M, a.dsum);
     ISAR_COUNT(1);
-    k_fe_phase<<<1, 1024, 0, st>>>(nullptr, 0, a.dsum, M, a.phase, a.fdec);
+    k_fe_phase<<<M / 32, M, 0, st>>>(nullptr, 0, a.dsum, M, a.phase, a.fdec);
     ISAR_COUNT(1);
     if (a.pre_only) return cudaGetLastError();
     if (a.ws_w && (a.af_cluster == 0 || a.iters == 0)) return cudaErrorInvalidValue;

@@ -926,6 +926,7 @@ __global__ void k_arp_reduce(const float* __restrict__ part, int nparts, int N, 
     const float invM = 1.0f / (float)M;
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         float s = 0.0f;
+#pragma unroll 16
         for (int p = 0; p < nparts; ++p) s += part[(size_t)p * N + n];
         arp[n] = (s * inv) * invM;
     }
@@ -948,6 +949,7 @@ __global__ void k_ycolsum(const float2* __restrict__ y, int N, int rows, float* 
 {
     for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
         float s = 0.0f;
+#pragma unroll 32
         for (int m = 0; m < rows; ++m) {
             const float2 v = y[(size_t)m * N + n];
             s += sqrtf(v.x * v.x + v.y * v.y);
@@ -973,119 +975,119 @@ __device__ __forceinline__ float arp_mean(const float* arp, int idx, int WL, int
     return s;
 }
 
-template <class T>
-__device__ __forceinline__ T block_sum_1024(T v, T* red)
+// Ascending sort of the n = 8 T unsigned keys that threads t < T hold (thread
+// t: elements 8 t .. 8 t + 7 of the current order), one CTA; T a multiple of
+// 32.  An LSD radix sort on 4-bit digits: every thread counts its keys in
+// counters of its own (digits d and d + 8 share a word, so a pass has 8 T words
+// and no thread waits for another), the packed counters are scanned in (digit,
+// thread) order, and the keys are exchanged through sm.  Passes run over the
+// bits up to `bits` only.  sm, cnt: 8 T words each, 16-byte aligned; red: 32
+// words.  The keys end in sm in order (and in k).
+// One CTA, bound by shared memory: 37800 clocks at 8192 keys and 22100 at 4096,
+// where four 8-bit passes ranked by warp matches took 66200 and 38300.
+__device__ void block_radix_sort(unsigned (&k)[8], unsigned* sm, unsigned* cnt, unsigned* red, int T, int bits)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if (lane == 0) red[w] = v;
-    __syncthreads();
-    if (w == 0) {
-        v = (lane < (int)(blockDim.x >> 5)) ? red[lane] : (T)0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[0] = v;
-    }
-    __syncthreads();
-    v = red[0];
-    __syncthreads();
-    return v;
-}
-
-// Ascending sort of the n non-negative floats in s (their bit patterns order
-// as unsigned integers), one CTA of 1024 threads: an LSD radix sort, four
-// passes of 8-bit digits.  Threads t < n / 8 (whole warps, n >= 256) hold 8
-// keys each; slot e of lane l of warp w is element 256 w + 32 e + l of the
-// current order, which every pass keeps stable: within a warp a key's rank
-// among equal digits comes from __match_any_sync and a running count per
-// (digit, warp) over the slots, across warps from an exclusive scan of the
-// counts in digit-major order.  cnt: 256 * (n / 256 + 1) ints (one pad
-// column against bank conflicts); red: 32 ints.
-__device__ void block_radix_sort(float* s, int n, int* cnt, int* red)
-{
-    const int T = n / 8, W = T / 32, WP = W + 1;
-    const int lw = 31 - __clz(W);   // W = n / 256 is a power of two
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const bool act = tid < T;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    unsigned k[8];
-    int off[8];
+    const bool act = tid < T;   // whole warps
+    uint4* sm4 = reinterpret_cast<uint4*>(sm);
+    uint4* cnt4 = reinterpret_cast<uint4*>(cnt);
+    uint16_t* c16 = reinterpret_cast<uint16_t*>(cnt);
 #pragma unroll 1
-    for (int shift = 0; shift < 32; shift += 8) {
-        for (int i = tid; i < 256 * WP; i += blockDim.x) cnt[i] = 0;
+    for (int shift = 0; shift < bits; shift += 4) {
+        int off[8], at[8];
+        unsigned x[8], incl = 0, sum = 0;
         if (act) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) k[e] = __float_as_uint(s[256 * w + 32 * e + lane]);
-        }
-        __syncthreads();   // keys loaded, counters cleared
-        if (act) {
+            for (int d = 0; d < 8; ++d) cnt[d * T + tid] = 0;
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
-                const int d = (int)((k[e] >> shift) & 255u);
-                const unsigned peers = __match_any_sync(0xffffffffu, d);
-                const int rank = __popc(peers & lt_mask);
-                const int base = cnt[d * WP + w];
-                off[e] = base + rank;
-                __syncwarp();
-                if (rank == 0) cnt[d * WP + w] = base + __popc(peers);
-                __syncwarp();
+                const unsigned d = (k[e] >> shift) & 15u;
+                at[e] = (int)(((d & 7u) * T + tid) * 2 + (d >> 3));
+                off[e] = c16[at[e]];
+                c16[at[e]] = (uint16_t)(off[e] + 1);
             }
         }
         __syncthreads();
-        // exclusive scan of cnt over f = d * W + w: q consecutive entries per
-        // thread, then the threads' totals across the block
-        const int total = 256 * W;
-        const int q = (total + (int)blockDim.x - 1) / (int)blockDim.x;   // <= 8
-        const int f0 = tid * q;
-        int loc[8];
-        int sum = 0;
+        if (act) {
+            const uint4 p = cnt4[2 * tid], q = cnt4[2 * tid + 1];
+            x[0] = p.x, x[1] = p.y, x[2] = p.z, x[3] = p.w, x[4] = q.x, x[5] = q.y, x[6] = q.z, x[7] = q.w;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            loc[j] = sum;
-            const int f = f0 + j;
-            if (j < q && f < total) sum += cnt[(f >> lw) * WP + (f & (W - 1))];
-        }
-        int x = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) red[w] = x;
-        __syncthreads();
-        if (w == 0) {
-            const int v = lane < (int)(blockDim.x >> 5) ? red[lane] : 0;
-            int z = v;
+            for (int j = 0; j < 8; ++j) {   // exclusive within the thread
+                const unsigned v = x[j];
+                x[j] = sum;
+                sum += v;
+            }
+            incl = sum;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, z, o);
+                const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            if (lane == 31) red[w] = incl;
+        }
+        __syncthreads();
+        if (act) {
+            unsigned z = lane < (T >> 5) ? red[lane] : 0u;   // every warp scans the warps' totals
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned y = __shfl_up_sync(0xffffffffu, z, o);
                 if (lane >= o) z += y;
             }
-            red[lane] = z - v;
+            const unsigned total = __shfl_sync(0xffffffffu, z, 31);
+            const unsigned before = __shfl_sync(0xffffffffu, z, w == 0 ? 0 : w - 1);
+            // digits 8..15 follow all of 0..7
+            const unsigned base = (w == 0 ? 0u : before) + incl - sum + (total << 16);
+            cnt4[2 * tid] = make_uint4(x[0] + base, x[1] + base, x[2] + base, x[3] + base);
+            cnt4[2 * tid + 1] = make_uint4(x[4] + base, x[5] + base, x[6] + base, x[7] + base);
         }
         __syncthreads();
-        const int excl = red[w] + x - sum;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int f = f0 + j;
-            if (j < q && f < total) cnt[(f >> lw) * WP + (f & (W - 1))] = excl + loc[j];
-        }
-        __syncthreads();   // cnt holds each (digit, warp) start
         if (act) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const int d = (int)((k[e] >> shift) & 255u);
-                s[cnt[d * WP + w] + off[e]] = __uint_as_float(k[e]);
-            }
+            for (int e = 0; e < 8; ++e) sm[c16[at[e]] + off[e]] = k[e];
         }
         __syncthreads();
+        if (act) {
+            const uint4 p = sm4[2 * tid], q = sm4[2 * tid + 1];
+            k[0] = p.x, k[1] = p.y, k[2] = p.z, k[3] = p.w, k[4] = q.x, k[5] = q.y, k[6] = q.z, k[7] = q.w;
+        }
+    }
+}
+
+// The best (value, index) pair of the CTA in every thread: `better` orders
+// them; red: 32 pairs.
+template <class Better>
+__device__ __forceinline__ void block_best(float& v, int& i, float2* red, Better better)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+        if (better(ov, oi, v, i)) {
+            v = ov;
+            i = oi;
+        }
+    }
+    if (lane == 0) red[w] = make_float2(v, __int_as_float(i));
+    __syncthreads();
+    const float2 r = red[lane < (int)(blockDim.x >> 5) ? lane : 0];
+    v = r.x;
+    i = __float_as_int(r.y);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, v, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, i, o);
+        if (better(ov, oi, v, i)) {
+            v = ov;
+            i = oi;
+        }
     }
 }
 
 // HRRPCenter decisions + cutRangeProfile offset, one CTA of 1024 threads.
 // dec: [0] applied, [1] shift_num, [2] cut offset, [3] |idx_1|, [4] |idx_2|,
 //      [5] threshold (float bits).
+// Dynamic shared memory: 3 N words (profile, sorted profile, sort counters).
 __global__ void __launch_bounds__(1024)
 k_center(const float* __restrict__ arp_g, const float2* __restrict__ y, int N, int inter_length,
          int* __restrict__ dec)
@@ -1093,21 +1095,43 @@ k_center(const float* __restrict__ arp_g, const float2* __restrict__ y, int N, i
     extern __shared__ float4 dyn_smem[];
     float* arp = reinterpret_cast<float*>(dyn_smem);
     float* srt = arp + N;
-    __shared__ long long red_ll[32];
-    __shared__ int red_i[32];
-    __shared__ float red_f[32];
-    __shared__ int red_j[32];
-    __shared__ int sort_cnt[256 * (kMaxN / 256 + 1)];
-    const int tid = threadIdx.x;
-    for (int i = tid; i < N; i += blockDim.x) {
-        const float v = arp_g[i];
-        arp[i] = v;
-        srt[i] = v;
+    unsigned* cnt = reinterpret_cast<unsigned*>(srt + N);
+    __shared__ unsigned red_u[32];
+    __shared__ float2 red_a[32], red_b[32];
+    __shared__ int red_sum[32];
+    __shared__ int2 red_n[32];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int T = N / 8;
+    // the profile, 8 consecutive cells per thread, and |Re| + |Im| of row 0
+    // (for the cut below: its load overlaps the sort)
+    unsigned k[8];
+    float mag[8];
+    unsigned top = 0;
+    if (tid < T) {
+        const float4 p = reinterpret_cast<const float4*>(arp_g)[2 * tid];
+        const float4 q = reinterpret_cast<const float4*>(arp_g)[2 * tid + 1];
+        reinterpret_cast<float4*>(arp)[2 * tid] = p;
+        reinterpret_cast<float4*>(arp)[2 * tid + 1] = q;
+        const float f[8] = {p.x, p.y, p.z, p.w, q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float2 v = y[tid + e * T];
+            mag[e] = fabsf(v.x) + fabsf(v.y);
+            k[e] = __float_as_uint(f[e]);   // non-negative floats order as their bits
+            top |= k[e];
+        }
     }
+    // bits that any key uses (the sort's passes)
+    top = __reduce_or_sync(0xffffffffu, top);
+    if (lane == 0) red_u[w] = top;
     __syncthreads();
+    top = __reduce_or_sync(0xffffffffu, red_u[lane]);
     // ascending sort (thrust::stable_sort of arp1, :404; values only, so
     // stability does not show)
-    block_radix_sort(srt, N, sort_cnt, red_i);
+    block_radix_sort(k, reinterpret_cast<unsigned*>(srt), cnt, red_u, T, 32 - __clz(top));
+    if (top == 0 && tid < T)   // no pass ran: all keys are zero
+        for (int e = 0; e < 8; ++e) srt[8 * tid + e] = 0.0f;
+    __syncthreads();
     // extra = inter_length * max(arp1) / N ; diff argmin (first index) (:406-420)
     const float arp1_max = srt[N - 1];
     const float extra = (float)inter_length * arp1_max / (float)N;
@@ -1121,38 +1145,13 @@ k_center(const float* __restrict__ arp_g, const float2* __restrict__ y, int N, i
             bi = i;
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov < bv || (ov == bv && oi < bi)) {
-            bv = ov;
-            bi = oi;
-        }
-    }
-    if ((tid & 31) == 0) {
-        red_f[tid >> 5] = bv;
-        red_j[tid >> 5] = bi;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        float v = red_f[0];
-        int ii = red_j[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            if (red_f[w] < v || (red_f[w] == v && red_j[w] < ii)) {
-                v = red_f[w];
-                ii = red_j[w];
-            }
-        red_j[0] = ii;
-    }
-    __syncthreads();
+    block_best(bv, bi, red_a, [](float av, int ai, float cv, int ci) { return av < cv || (av == cv && ai < ci); });
     // a profile without a finite minimum (NaN everywhere) keeps index 0
-    const int dmin = red_j[0] < dl ? red_j[0] : 0;
-    __syncthreads();
+    const int dmin = bi < dl ? bi : 0;
     const float thr = srt[dmin + inter_length / 2];
     // idx_1 = find(arp > thr); drop those whose 9-tap mean < thr (:426-449)
     int n1 = 0, n2 = 0;
-    long long sum = 0;
+    int sum = 0;   // at most 8 indices per thread and 256 per warp: below 2^31
     for (int n = tid; n < N; n += blockDim.x) {
         if (arp[n] > thr) {
             ++n1;
@@ -1160,49 +1159,43 @@ k_center(const float* __restrict__ arp_g, const float2* __restrict__ y, int N, i
             else sum += n;
         }
     }
-    n1 = block_sum_1024<int>(n1, red_i);
-    n2 = block_sum_1024<int>(n2, red_i);
-    sum = block_sum_1024<long long>(sum, red_ll);
+    n1 = __reduce_add_sync(0xffffffffu, n1);
+    n2 = __reduce_add_sync(0xffffffffu, n2);
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) {
+        red_n[w] = make_int2(n1, n2);
+        red_sum[w] = sum;
+    }
+    __syncthreads();
+    {
+        const int2 r = red_n[lane];
+        n1 = __reduce_add_sync(0xffffffffu, r.x);
+        n2 = __reduce_add_sync(0xffffffffu, r.y);
+        sum = __reduce_add_sync(0xffffffffu, red_sum[lane]);   // below N^2 / 2 = 2^25
+    }
     int applied = 0, shift = 0;
     if (n2 != n1) {
-        const int mean_idx = (int)(sum / (long long)(n1 - n2));
+        const int mean_idx = sum / (n1 - n2);
         shift = -(mean_idx - N / 2);
         applied = 1;
     }
-    // cutRangeProfile: Icamax (|Re|+|Im|, first max) of centred row 0
+    // cutRangeProfile: Icamax (|Re|+|Im|, first max) of centred row 0, whose
+    // cell n is cell n - shift of row 0
     float cv = -1.0f;
     int ci = 0x7fffffff;
-    for (int n = tid; n < N; n += blockDim.x) {
-        const float2 v = y[(n - shift) & (N - 1)];
-        const float a = fabsf(v.x) + fabsf(v.y);
-        if (a > cv) {
-            cv = a;
-            ci = n;
-        }
-    }
+    if (tid < T) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, cv, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, ci, o);
-        if (ov > cv || (ov == cv && oi < ci)) {
-            cv = ov;
-            ci = oi;
+        for (int e = 0; e < 8; ++e) {
+            const int n = (tid + e * T + shift) & (N - 1);
+            if (mag[e] > cv || (mag[e] == cv && n < ci)) {
+                cv = mag[e];
+                ci = n;
+            }
         }
     }
-    if ((tid & 31) == 0) {
-        red_f[tid >> 5] = cv;
-        red_j[tid >> 5] = ci;
-    }
-    __syncthreads();
+    block_best(cv, ci, red_b, [](float av, int ai, float bv_, int bi_) { return av > bv_ || (av == bv_ && ai < bi_); });
     if (tid == 0) {
-        float v = red_f[0];
-        int ii = red_j[0];
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            if (red_f[w] > v || (red_f[w] == v && red_j[w] < ii)) {
-                v = red_f[w];
-                ii = red_j[w];
-            }
-        int off = ii - kRangeCut / 2;
+        int off = ci - kRangeCut / 2;
         if (off < 0) off = 0;
         if (off > N - kRangeCut) off = N - kRangeCut;
         dec[0] = applied;
@@ -1473,7 +1466,7 @@ cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec
     static PerDevice attr;   // k_center's shared-memory limit, set once per device
     const int ar = attr.get([]() -> int { return -(int)center_prepare_current_device(); });
     if (ar < 0) return (cudaError_t)(-ar);
-    k_center<<<1, 1024, 2 * N * sizeof(float), st>>>(arp, y, N, 30, dec);
+    k_center<<<1, 1024, 3 * N * sizeof(float), st>>>(arp, y, N, 30, dec);
     ISAR_COUNT(1);
     k_cut<<<M, 256, 0, st>>>(y, N, dec, cut);
     ISAR_COUNT(1);
@@ -1482,7 +1475,7 @@ cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec
 
 cudaError_t center_prepare_current_device()
 {
-    return cudaFuncSetAttribute(k_center, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMaxN * (int)sizeof(float));
+    return cudaFuncSetAttribute(k_center, cudaFuncAttributeMaxDynamicSharedMemorySize, 3 * kMaxN * (int)sizeof(float));
 }
 
 template <int N>
