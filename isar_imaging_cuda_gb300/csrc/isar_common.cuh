@@ -57,6 +57,19 @@ __device__ __forceinline__ float2 csub(float2 a, float2 b)
     asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2u(a)), "l"(f2u(b)));
     return u2f(r);
 }
+// Componentwise product and fused multiply-add of packed pairs.
+__device__ __forceinline__ float2 pmul(float2 a, float2 b)
+{
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(f2u(a)), "l"(f2u(b)));
+    return u2f(r);
+}
+__device__ __forceinline__ float2 pfma(float2 a, float2 b, float2 c)
+{
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(f2u(a)), "l"(f2u(b)), "l"(f2u(c)));
+    return u2f(r);
+}
 __device__ __forceinline__ float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 __device__ __forceinline__ float cabs2(float2 a) { return a.x * a.x + a.y * a.y; }
 __device__ __forceinline__ float2 conjf2(float2 a) { return make_float2(a.x, -a.y); }

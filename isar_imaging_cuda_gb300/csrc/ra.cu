@@ -195,11 +195,16 @@ __global__ void k_zero_shift(double* __restrict__ S, int64_t* __restrict__ SQ, i
 // S[row] += sh and SQ[row] = S[row] / N as a 64-bit fixed-point fraction,
 // once per row (one thread), so that the row transforms read SQ directly.
 template <int N>
-__device__ __forceinline__ void add_shift(double* S, int64_t* SQ, size_t row, float sh)
+__device__ __forceinline__ void add_shift_to(double* S, int64_t* SQ, size_t row, double before, float sh)
 {
-    const double v = S[row] + (double)sh;
+    const double v = before + (double)sh;
     S[row] = v;
     SQ[row] = cells_to_fixed((uint64_t)__double_as_longlong(v), ilog2c(N));
+}
+template <int N>
+__device__ __forceinline__ void add_shift(double* S, int64_t* SQ, size_t row, float sh)
+{
+    add_shift_to<N>(S, SQ, row, S[row], sh);
 }
 
 // The slope SQ of one shift sh.
@@ -254,15 +259,16 @@ __device__ __forceinline__ ArgKey block_argmax(ArgKey k, ArgKey* red)
     return k;
 }
 
-// Error-free float accumulation (TwoSum) of the exact product a*b (TwoProd via
-// FMA) into the pair (hi, lo).
-__device__ __forceinline__ void acc_prod(float a, float b, float& hi, float& lo)
+// Error-free float accumulation (TwoSum) of the exact products a*b (TwoProd via
+// FMA) into the pairs (hi, lo), two independent sums in packed pairs;
+// na = -a.
+__device__ __forceinline__ void acc_prod(float2 a, float2 na, float2 b, float2& hi, float2& lo)
 {
-    const float p = a * b;
-    const float e = fmaf(a, b, -p);
-    const float t = hi + p;
-    const float z = t - hi;
-    lo += (hi - (t - z)) + (p - z) + e;
+    const float2 np = pmul(na, b);   // -p
+    const float2 e = pfma(a, b, np);
+    const float2 t = csub(hi, np);
+    const float2 z = csub(t, hi);
+    lo = cadd(lo, cadd(csub(csub(hi, csub(t, z)), cadd(np, z)), e));
     hi = t;
 }
 
@@ -275,34 +281,36 @@ __device__ __forceinline__ void pair_add(float& h, float& l, float h2, float l2)
     h = t;
 }
 
-// Block totals of three compensated float pairs as floats, valid in threads
-// 0, 1 and 2 (total j in thread j); one barrier.  Float arithmetic throughout
-// with the precision of a double sum (FP64 issues slowly on this part: only
-// the final rounding of the three totals uses it, in one warp).
+// Block totals of three compensated float pairs as floats, total j in lane 0
+// of warp j (in warp 0 for a block of one or two warps, lane j); two barriers,
+// the second after the totals are in s_f.  Float arithmetic throughout with
+// the precision of a double sum (FP64 issues slowly on this part: only the
+// final rounding of the three totals uses it, in one lane each).
 template <int T>
-__device__ __forceinline__ float block_sum_pair3(float* h, float* l, float2 (*red)[32])
+__device__ __forceinline__ void block_sum_pair3(float* h, float* l, float2 (*red)[32], float* s_f)
 {
+    constexpr int W = T / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
             pair_add(h[j], l[j], __shfl_xor_sync(0xffffffffu, h[j], o), __shfl_xor_sync(0xffffffffu, l[j], o));
     }
-    constexpr int W = T / 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    if constexpr (W > 1) {
-        if (lane < 3) red[lane][w] = make_float2(lane == 0 ? h[0] : lane == 1 ? h[1] : h[2],
-                                                 lane == 0 ? l[0] : lane == 1 ? l[1] : l[2]);
-        __syncthreads();
+    if (lane < 3)
+        red[lane][w] = make_float2(lane == 0 ? h[0] : lane == 1 ? h[1] : h[2],
+                                   lane == 0 ? l[0] : lane == 1 ? l[1] : l[2]);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        if (w != (W >= 3 ? j : 0)) continue;
+        float2 v = lane < W ? red[j][lane] : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int o = W / 2; o > 0; o >>= 1)
+            pair_add(v.x, v.y, __shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o));
+        if (lane == 0) s_f[j] = (float)((double)v.x + (double)v.y);
     }
-    float r = 0.0f;
-    if (w == 0 && lane < 3) {
-        float H = lane == 0 ? h[0] : lane == 1 ? h[1] : h[2], L = lane == 0 ? l[0] : lane == 1 ? l[1] : l[2];
-#pragma unroll 1
-        for (int i = 1; i < W; ++i) pair_add(H, L, red[lane][i].x, red[lane][i].y);
-        r = (float)((double)H + (double)L);
-    }
-    return r;
+    __syncthreads();
 }
 
 // float(hi + lo + x) for a compensated pair (|lo| <= ulp(hi)), rounded once
@@ -341,6 +349,7 @@ __device__ RaShift ra_correlate_f(AmpA A, AmpB B, float* sm_f, int lt, const Tw&
     float2* sm = reinterpret_cast<float2*>(sm_f);
     __shared__ ArgKey red[32];
     __shared__ float2 redp[3][32];
+    __shared__ float s_f[3];
     __shared__ RaShift s_res;
     // z = a + i b, forward FFT, spectrum kept in the scratch (padded slots)
     team_fft<N, false>([&](int i) { return make_float2(A(i), B(i)); },
@@ -371,30 +380,41 @@ __device__ RaShift ra_correlate_f(AmpA A, AmpB B, float* sm_f, int lt, const Tw&
     const int pos = block_argmax<T>(best, red).i;
     const int tau = (pos + N / 2) & (N - 1);
     // f_j = sum_n a[n] b[n - (tau + j)], j = -1, 0, 1
-    float h[3] = {0.0f, 0.0f, 0.0f}, l[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll 4
-    for (int t = 0; t < N / T; ++t) {
-        const int n = lt + t * T;
-        const float a = A(n);
+    float h[3], l[3];
+    {
+        float2 h2[3], l2[3];   // even and odd t
 #pragma unroll
-        for (int j = 0; j < 3; ++j) acc_prod(a, B((n - tau - (j - 1)) & (N - 1)), h[j], l[j]);
+        for (int j = 0; j < 3; ++j) h2[j] = l2[j] = make_float2(0.0f, 0.0f);
+#pragma unroll 4
+        for (int t = 0; t < N / T; t += 2) {
+            const int n = lt + t * T;
+            const float2 a = make_float2(A(n), A(n + T)), na = make_float2(-a.x, -a.y);
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                const int k = n - tau - (j - 1);
+                acc_prod(a, na, make_float2(B(k & (N - 1)), B((k + T) & (N - 1))), h2[j], l2[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            h[j] = h2[j].x;
+            l[j] = l2[j].x;
+            pair_add(h[j], l[j], h2[j].y, l2[j].y);
+        }
     }
-    const float f = block_sum_pair3<T>(h, l, redp);
-    if (lt < 32) {
+    block_sum_pair3<T>(h, l, redp, s_f);
+    if (lt == 0) {
         // the reference keeps the correlation in a float buffer and fits the
         // parabola in float (binomialFixDevice, range_alignment.cu:121-131)
-        const float f1 = __shfl_sync(0xffffffffu, f, 0), f2 = __shfl_sync(0xffffffffu, f, 1),
-                    f3 = __shfl_sync(0xffffffffu, f, 2);
+        const float f1 = s_f[0], f2 = s_f[1], f3 = s_f[2];
         const float fa = __fdiv_rn(__fsub_rn(__fadd_rn(f1, f3), __fmul_rn(2.0f, f2)), 2.0f);
         const float fb = __fdiv_rn(__fsub_rn(f3, f1), 2.0f);
         const float delta = __fdiv_rn(-fb, __fmul_rn(2.0f, fa));
         float sh = __fsub_rn(__fadd_rn((float)pos, delta), (float)N / 2);
         if (given) sh = *shift_out;   // injected by the caller (test hook)
-        if (lt == 0) {
-            if (!given) *shift_out = sh;
-            s_res.sh = sh;
-            s_res.slope = shift_slope<N>(sh);
-        }
+        else *shift_out = sh;
+        s_res.sh = sh;
+        s_res.slope = shift_slope<N>(sh);
     }
     __syncthreads();
     return s_res;
@@ -801,6 +821,10 @@ k_ra_spec(const float2* __restrict__ wprev, float2* __restrict__ wout, double* _
     float2* sm = reinterpret_cast<float2*>(sm_f);
     const int lt = threadIdx.x, j = blockIdx.x;
     const int s = 1 << level;
+    // the shifts of the second group's rows: read here, where the load's
+    // latency is hidden, written at the end
+    const size_t row2 = (size_t)(2 * j + 1) * s + lt;
+    const double s_old = lt < s ? S[row2] : 0.0;
     RaTw<N>::fill(twt, tw, lt, F::T);
     __syncthreads();
     const RaTw<N> tws{twt};
@@ -825,7 +849,8 @@ k_ra_spec(const float2* __restrict__ wprev, float2* __restrict__ wout, double* _
     __syncthreads();
     const auto [sh, slope] = ra_correlate_f<N>([&](int n) { return ea[n]; }, [&](int n) { return eb[n]; }, sm_f, lt,
                                                tws, shift_out + j, given);
-    for (int m = lt; m < s; m += F::T) add_shift<N>(S, SQ, (size_t)(2 * j + 1) * s + m, sh);
+    if (lt < s) add_shift_to<N>(S, SQ, row2, s_old, sh);
+    for (int m = lt + F::T; m < s; m += F::T) add_shift<N>(S, SQ, (size_t)(2 * j + 1) * s + m, sh);
     if (wout == nullptr) return;
     LinPhase<N> r;
     r.init(slope, lt);
