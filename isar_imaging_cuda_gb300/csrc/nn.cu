@@ -54,10 +54,11 @@ __global__ void k_im2col(const __nv_bfloat16* __restrict__ act, int frames, int 
 
 // Per frame: delta_m = atan2(s, c) - r_m (m < M-1), z = mean exp(j delta),
 // loss = 1 - |z|; d loss / d r_hat_m = Im(conj(z) exp(j delta_m)) / ((M-1) |z|)
-// / frames, chained through r_hat = atan2(s, c) into dout (bf16 [rows][16]).
+// / frames, chained through r_hat = atan2(s, c) into dout (bf16 [rows][ld], ld
+// a multiple of 8, zero past the two columns).
 __global__ void __launch_bounds__(256)
 k_loss(const float* __restrict__ out, const float* __restrict__ target, int M, int frames, float* __restrict__ loss,
-       __nv_bfloat16* __restrict__ dout)
+       __nv_bfloat16* __restrict__ dout, int ld)
 {
     const int b = blockIdx.x;
     const int tid = threadIdx.x;
@@ -109,10 +110,10 @@ k_loss(const float* __restrict__ out, const float* __restrict__ target, int M, i
             dc = -g * s / r2;
             ds = g * c / r2;
         }
-        dout[p * kOutPad] = __float2bfloat16_rn(dc);
-        dout[p * kOutPad + 1] = __float2bfloat16_rn(ds);
-#pragma unroll
-        for (int q = 2; q < kOutPad; ++q) dout[p * kOutPad + q] = __float2bfloat16_rn(0.0f);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(dc, ds);
+        uint4* row = reinterpret_cast<uint4*>(dout + p * ld);
+        row[0] = make_uint4(*reinterpret_cast<const uint32_t*>(&h), 0u, 0u, 0u);
+        for (int q = 1; q < ld / 8; ++q) row[q] = make_uint4(0u, 0u, 0u, 0u);
     }
 }
 
@@ -368,11 +369,20 @@ cudaError_t forward(const Weights& w, Acts& a, int frames, int M, int* err, cuda
         ep.ld_bf16 = kCh;
         return ep;
     };
+    const bool implicit = M % 128 == 0;
+    a.have_cols = a.cols[0] && !implicit;
+    if (a.cols[0] && implicit) {
+        // training: the backward pass reads X0 too, and the caller may reuse
+        // its buffer after this call
+        if ((e = cudaMemcpyAsync(a.cols[0], a.act[0], (size_t)rows * kCh * sizeof(__nv_bfloat16),
+                                 cudaMemcpyDeviceToDevice, st)))
+            return e;
+        a.act[0] = a.cols[0];
+    }
     for (int l = 0; l < kConv; ++l) {
-        if (!a.cols[l] && M % 128 == 0) {
-            // inference: the conv's im2col operand read tap by tap from the
-            // activations by the GEMM itself (training keeps the columns for
-            // the weight gradients)
+        if (implicit) {
+            // the conv's im2col operand is read tap by tap from the
+            // activations by the GEMM itself
             GemmConvA cv;
             cv.act = a.act[l];
             cv.frames = frames;
@@ -427,8 +437,39 @@ cudaError_t backward(const Weights& w, Acts& a, Grads& g, const float* target, i
     const long rows = (long)frames * M;
     cudaError_t e;
     if ((e = cudaMemsetAsync(g.g, 0, (size_t)kParams * sizeof(float), st))) return e;
+    if (M % 128 == 0 && !a.have_cols) {
+        // two kernels per layer, reading activations and dz where they lie
+        // (nn_gemm.cu); dz alternates between two buffers
+        __nv_bfloat16 *dz = g.dz, *dz2 = g.dzT;
+        k_loss<<<frames, 256, 0, st>>>(a.out, target, M, frames, g.loss, dz, kCh);
+        ISAR_COUNT(1);
+        for (int l = kConv + 1; l >= 0; --l) {
+            const int taps = l < kConv ? kTaps : 1;
+            const int nout = w_rows(l);
+            if ((e = layer_wgrad(taps, a.act[l], dz, g.g + w_off(l), g.g + b_off(l), nout, frames, M, err, st)))
+                return e;
+            if (l == 0) break;
+            if ((e = layer_dgrad(taps, dz, w.wt[l], l == kConv + 1 ? kOutPad : kCh, a.act[l], dz2, frames, M, err, st)))
+                return e;
+            std::swap(dz, dz2);
+        }
+        return cudaGetLastError();
+    }
+    if (!a.have_cols) {   // the last forward's frame length needed none
+        for (int l = 0; l < kConv; ++l) {
+            if (l == 0 && a.act[0] == a.cols[0]) {   // X0's copy lies where the columns go
+                if ((e = cudaMemcpyAsync(g.colT, a.cols[0], (size_t)rows * kCh * sizeof(__nv_bfloat16),
+                                         cudaMemcpyDeviceToDevice, st)))
+                    return e;
+            }
+            k_im2col<<<grid_for(rows * kTaps * (kCh / 8), 256), 256, 0, st>>>(
+                l == 0 && a.act[0] == a.cols[0] ? g.colT : a.act[l], frames, M, a.cols[l]);
+            ISAR_COUNT(1);
+        }
+        a.have_cols = true;
+    }
     // output layer: dout (bf16 [rows][16]) into g.dz
-    k_loss<<<frames, 256, 0, st>>>(a.out, target, M, frames, g.loss, g.dz);
+    k_loss<<<frames, 256, 0, st>>>(a.out, target, M, frames, g.loss, g.dz, kOutPad);
     ISAR_COUNT(1);
     const int cs_grid = (int)std::min<long>(rows, 1024);
     k_colsum<<<cs_grid, kOutPad, 0, st>>>(g.dz, rows, kOutPad, 2, g.g + b_off(kConv + 1));

@@ -47,7 +47,9 @@ struct Acts {
     int rows = 0;
     __nv_bfloat16* act[kConv + 2] = {};       // act[0] = X0 (caller-filled), act[l+1] = layer l output [rows][64]
     __nv_bfloat16* col = nullptr;             // [rows][320] im2col scratch (inference) or
-    __nv_bfloat16* cols[kConv] = {};          // per conv layer (training keeps them for the weight gradients)
+    __nv_bfloat16* cols[kConv] = {};          // per conv layer, training (M not a multiple of 128; otherwise
+                                              // cols[0] holds a copy of X0)
+    bool have_cols = false;                   // the last forward filled cols[]
     float* out = nullptr;                     // [rows][16] network output (c, s, 14 pad)
 };
 
@@ -77,11 +79,23 @@ cudaError_t gemm_tn(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int
                     int Nc, int K, int splits, int* err, cudaStream_t st, const GemmEpilogue& ep = GemmEpilogue{},
                     const GemmConvA& conv = GemmConvA{});
 
+// Backward pass of one layer of `taps` (5 or 1) x 64 channels, M a multiple of
+// 128.  layer_dgrad: dz_out = bf16(act > 0 ? input gradient : 0) from dz and the
+// layer's transposed weights wt [taps*64][wt_cols] (dz columns past wt_cols are
+// not read); dz_out must not be dz.  layer_wgrad: adds the weight gradient
+// ([nout][taps*64]) and the bias gradient ([nout]) into gw and gb.  All row
+// operands are [frames][M][64] bf16.
+cudaError_t layer_dgrad(int taps, const __nv_bfloat16* dz, const __nv_bfloat16* wt, int wt_cols,
+                        const __nv_bfloat16* act, __nv_bfloat16* dz_out, int frames, int M, int* err, cudaStream_t st);
+cudaError_t layer_wgrad(int taps, const __nv_bfloat16* act, const __nv_bfloat16* dz, float* gw, float* gb, int nout,
+                        int frames, int M, int* err, cudaStream_t st);
+
 // Refreshes the bf16 copies (and transposes) from the fp32 master.
 cudaError_t refresh_bf16(const Weights& w, cudaStream_t st);
 
-// Forward over frames x M positions; act[0] must hold X0.  Keeps every
-// layer's im2col when a.cols[] are set (training).
+// Forward over frames x M positions; act[0] must hold X0.  With a.cols[] set
+// (training) it keeps what the backward pass reads: a copy of X0 (M a multiple
+// of 128; act[0] then points to it) or every layer's im2col.
 cudaError_t forward(const Weights& w, Acts& a, int frames, int M, int* err, cudaStream_t st);
 
 // Training buffers for the backward pass.

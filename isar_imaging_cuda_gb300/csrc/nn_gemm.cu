@@ -333,16 +333,16 @@ static cudaError_t operand_map(CUtensorMap* m, const __nv_bfloat16* p, int rows,
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
-// Tensor map of act [frames][M][64] bf16 in boxes of 64 x 128 x 1 with the
-// 128-byte swizzle (the implicit convolution's A operand).
-static cudaError_t conv_map(CUtensorMap* m, const __nv_bfloat16* act, int frames, int M)
+// Tensor map of act [frames][M][64] bf16 in boxes of 64 x box_rows x 1 with
+// the 128-byte swizzle (the implicit convolution's A operand: 128 rows).
+static cudaError_t rows_map(CUtensorMap* m, const __nv_bfloat16* act, int frames, int M, int box_rows)
 {
     const PFN_cuTensorMapEncodeTiled_v12000 fn = encode_tiled();
     if (!fn) return cudaErrorNotSupported;
     const cuuint64_t dims[3] = {(cuuint64_t)BK, (cuuint64_t)M, (cuuint64_t)frames};
     const cuuint64_t strides[2] = {(cuuint64_t)BK * sizeof(__nv_bfloat16),
                                    (cuuint64_t)M * BK * sizeof(__nv_bfloat16)};
-    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)BM, 1};
+    const cuuint32_t box[3] = {(cuuint32_t)BK, (cuuint32_t)box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<__nv_bfloat16*>(act), dims, strides, box,
                           estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -402,7 +402,7 @@ cudaError_t gemm_tn(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int
     CUtensorMap ma, mb;
     cudaError_t e;
     if (conv.act) {
-        if ((e = conv_map(&ma, conv.act, conv.frames, conv.M))) return e;
+        if ((e = rows_map(&ma, conv.act, conv.frames, conv.M, BM))) return e;
     } else if ((e = operand_map(&ma, A, Mr, K, lda, BM))) {
         return e;
     }
@@ -416,6 +416,368 @@ cudaError_t gemm_tn(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int
     if (e) return e;
     ISAR_COUNT(1);
     return cudaGetLastError();
+}
+
+// ---------------------------------------------------------------------------
+// Backward pass of a layer of TAPS taps x 64 channels (5: a convolution,
+// 1: a 1 x 1 layer) in two kernels that read the activations and the
+// pre-activation gradient dz ([frames][M][64] bf16) where they lie, instead
+// of through im2col, transposed copies, a [rows][320] gradient matrix, col2im
+// and separate mask, column-sum and scatter passes (8 launches and ~105 us per
+// convolution at 16384 rows; these two take ~21).  M is a multiple of 128, so that a
+// block of 64 or 128 rows lies in one frame; rows that a tap shifts out of the
+// frame are the tensor maps' zero fill.
+// ---------------------------------------------------------------------------
+constexpr int kTile = 64 * BK * 2;   // 64 x 64 bf16 (8 KB)
+
+// Input gradient of 128 rows and the mask of the layer below:
+//   dact[m][c] = sum_k sum_o dz[m - k + TAPS/2][o] W[o][k*64 + c],
+//   dz_out = bf16(act > 0 ? dact : 0).
+// One accumulator per tap: each is the sum over o that a row of the im2col
+// gradient holds, and the taps are added in their order, so the result is bit
+// for bit that of the GEMM and col2im.  All operands are in flight at once
+// (24 KB per tap): the kernel is bound by their latency.
+template <int TAPS>
+__global__ void __launch_bounds__(128, 1)
+k_dgrad(const __grid_constant__ CUtensorMap map_dz, const __grid_constant__ CUtensorMap map_wt,
+        const __nv_bfloat16* __restrict__ act, __nv_bfloat16* __restrict__ dz_out, int conv_M, int* err)
+{
+    constexpr int TCOLS = TAPS == 1 ? 64 : 512;
+    constexpr int kA = BM * BK * 2, kStep = kA + kTile;
+    static_assert(TAPS * 64 <= TCOLS, "one accumulator per tap");
+    extern __shared__ uint8_t gemm_smem[];
+    __shared__ __align__(8) uint64_t full[TAPS];
+    __shared__ __align__(8) uint64_t done;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int row0 = blockIdx.x * BM;
+    const uint32_t base = (smem_u32(gemm_smem) + 1023u) & ~1023u;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)),
+                     "n"(TCOLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int k = 0; k < TAPS; ++k) mbar_init(smem_u32(&full[k]));
+        mbar_init(smem_u32(&done));
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        s_fail = 0;
+        const int f = row0 / conv_M, m0 = row0 - f * conv_M;
+        for (int k = 0; k < TAPS; ++k) {
+            const uint32_t fb = smem_u32(&full[k]), sa = base + (uint32_t)(k * kStep);
+            mbar_expect_tx(fb, (uint32_t)kStep);
+            tma_load_3d(sa, &map_dz, 0, m0 + TAPS / 2 - k, f, fb);
+            tma_load_2d(sa + kA, &map_wt, 0, k * 64, fb);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    if (tid == 0) {
+        constexpr uint32_t idesc = idesc_bf16(BM, 64);
+        bool ok = true;
+        for (int k = 0; k < TAPS; ++k) {
+            if (!mbar_wait(smem_u32(&full[k]), 0u)) {   // the other copies are still waited for
+                ok = false;
+                continue;
+            }
+            if (!ok) continue;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t sa = base + (uint32_t)(k * kStep);
+#pragma unroll
+            for (int j = 0; j < BK / 16; ++j) {
+                const uint64_t ad = smem_desc_sw128(sa + 32 * j), bd = smem_desc_sw128(sa + kA + 32 * j);
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + (uint32_t)(k * 64)),
+                    "l"(ad), "l"(bd), "r"(idesc), "r"(j > 0 ? 1u : 0u)
+                    : "memory");
+            }
+        }
+        if (!ok) {
+            atomicExch(err, 1);
+            s_fail = 1;
+        }
+        umma_commit(smem_u32(&done));
+    }
+    __syncthreads();
+    if (!mbar_wait(smem_u32(&done), 0u)) {
+        atomicExch(err, 1);
+        s_fail = 1;
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (!s_fail) {
+        const size_t r = (size_t)row0 + warp * 32 + lane;
+#pragma unroll 1
+        for (int c0 = 0; c0 < kCh; c0 += 16) {
+            const uint4 m0 = *reinterpret_cast<const uint4*>(act + r * kCh + c0);
+            const uint4 m1 = *reinterpret_cast<const uint4*>(act + r * kCh + c0 + 8);
+            float sum[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) sum[j] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < TAPS; ++k) {
+                uint32_t v[16];
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                    "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                      "=r"(v[15])
+                    : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(k * 64 + c0))
+                    : "memory");
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum[j] += __uint_as_float(v[j]);
+            }
+            const uint32_t mk[8] = {m0.x, m0.y, m0.z, m0.w, m1.x, m1.y, m1.z, m1.w};
+            uint32_t pk[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&mk[j]);
+                const __nv_bfloat162 h = __floats2bfloat162_rn(__bfloat162float(a.x) > 0.0f ? sum[2 * j] : 0.0f,
+                                                               __bfloat162float(a.y) > 0.0f ? sum[2 * j + 1] : 0.0f);
+                pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+            }
+            uint4* dst = reinterpret_cast<uint4*>(dz_out + r * kCh + c0);
+            dst[0] = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            dst[1] = make_uint4(pk[4], pk[5], pk[6], pk[7]);
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TCOLS) : "memory");
+}
+
+// Descriptor of an MN-major tile: rows of 64 M (or N) elements along which K
+// advances, written by the tensor memory accelerator with the 128-byte
+// swizzle.  Leading offset: to the next 64 M elements (the next tile); stride:
+// 1024 B to the next 8 K rows.  A K step of 16 rows advances the start address
+// by 2048 bytes.
+__device__ __forceinline__ uint64_t smem_desc_mn_sw128(uint32_t saddr)
+{
+    return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(kTile >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) |
+           (1ull << 46) | (2ull << 61);
+}
+
+// Weight and bias gradients, added into g with atomics:
+//   gw[o*TAPS*64 + k*64 + c] += sum_p act[p + k - TAPS/2][c] dz[p][o],
+//   gb[o] += sum_p dz[p][o],   o < nout,
+// over blocks of 64 rows p, a contiguous range of them per CTA.  Both operands
+// have their rows as the contraction, so both tiles are MN-major as they lie
+// in memory (descriptor above; transpose bits in the instruction descriptor)
+// and no transposed copy is made.  A stage holds TAPS shifted activation
+// tiles, a tile of ones and the dz tile; two tiles make an MMA of M = 128, the
+// last tap pairs with the ones, whose product is the bias gradient.
+template <int TAPS>
+struct WgradSmem {
+    static constexpr int kTiles = TAPS + 2;
+    static constexpr int kStage = kTiles * kTile;
+    static constexpr int kRing = 3;
+    static constexpr size_t kBytes = 1024 + (size_t)kRing * kStage;
+};
+
+template <int TAPS>
+__global__ void __launch_bounds__(128, 1)
+k_wgrad(const __grid_constant__ CUtensorMap map_act, const __grid_constant__ CUtensorMap map_dz, float* __restrict__ gw,
+        float* __restrict__ gb, int nout, int nblocks, int per_cta, int conv_M, int* err)
+{
+    using S = WgradSmem<TAPS>;
+    constexpr int NP = (TAPS + 1) / 2;   // accumulators of 128 x 64
+    constexpr int TCOLS = NP * 64 <= 64 ? 64 : 256;
+    static_assert(TAPS % 2 == 1 && NP * 64 <= TCOLS, "the last tap pairs with the ones");
+    extern __shared__ uint8_t gemm_smem[];
+    __shared__ __align__(8) uint64_t full[S::kRing];
+    __shared__ __align__(8) uint64_t empty[S::kRing];
+    __shared__ __align__(8) uint64_t done;
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_fail;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int b0 = blockIdx.x * per_cta, nblk = min(per_cta, nblocks - b0);
+    const uint32_t pad = (1024u - (smem_u32(gemm_smem) & 1023u)) & 1023u;
+    const uint32_t base = smem_u32(gemm_smem) + pad;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)),
+                     "n"(TCOLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    if (tid == 0) {
+        for (int s = 0; s < S::kRing; ++s) {
+            mbar_init(smem_u32(&full[s]));
+            mbar_init(smem_u32(&empty[s]));
+        }
+        mbar_init(smem_u32(&done));
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+        s_fail = 0;
+    }
+    // the tiles of ones (bf16 0x3f80), once per stage
+    for (int s = 0; s < S::kRing; ++s) {
+        uint4* t = reinterpret_cast<uint4*>(gemm_smem + pad + s * S::kStage + TAPS * kTile);
+        for (int i = tid; i < kTile / 16; i += blockDim.x) t[i] = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = s_tmem;
+    if (tid == 0) {
+        constexpr uint32_t idesc = idesc_bf16(128, 64) | (1u << 15) | (1u << 16);   // A and B MN-major
+        auto load = [&](int b) {
+            const uint32_t fb = smem_u32(&full[b % S::kRing]), sa = base + (uint32_t)((b % S::kRing) * S::kStage);
+            const int p = (b0 + b) * 64, f = p / conv_M, m0 = p - f * conv_M;
+            mbar_expect_tx(fb, (uint32_t)((TAPS + 1) * kTile));
+            for (int k = 0; k < TAPS; ++k) tma_load_3d(sa + k * kTile, &map_act, 0, m0 + k - TAPS / 2, f, fb);
+            tma_load_3d(sa + (TAPS + 1) * kTile, &map_dz, 0, m0, f, fb);
+        };
+        int issued = 0, consumed = 0;
+        bool ok = true;
+        for (; issued < min(S::kRing - 1, nblk); ++issued) load(issued);
+        for (int b = 0; b < nblk; ++b) {
+            if (!mbar_wait(smem_u32(&full[b % S::kRing]), (uint32_t)((b / S::kRing) & 1))) {
+                ok = false;
+                break;
+            }
+            consumed = b + 1;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            const uint32_t sa = base + (uint32_t)((b % S::kRing) * S::kStage);
+#pragma unroll
+            for (int j = 0; j < 64 / 16; ++j) {
+                const uint64_t bd = smem_desc_mn_sw128(sa + (TAPS + 1) * kTile + 2048 * j);
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    const uint64_t ad = smem_desc_mn_sw128(sa + 2 * q * kTile + 2048 * j);
+                    asm volatile(
+                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + (uint32_t)(q * 64)),
+                        "l"(ad), "l"(bd), "r"(idesc), "r"(b > 0 || j > 0 ? 1u : 0u)
+                        : "memory");
+                }
+            }
+            umma_commit(smem_u32(&empty[b % S::kRing]));
+            // refill the stage of block b - 1 once its MMAs are done
+            const int nb = b + S::kRing - 1;
+            if (nb < nblk) {
+                if (nb >= S::kRing &&
+                    !mbar_wait(smem_u32(&empty[nb % S::kRing]), (uint32_t)((nb / S::kRing - 1) & 1))) {
+                    ok = false;
+                    break;
+                }
+                load(nb);
+                issued = nb + 1;
+            }
+        }
+        if (!ok) {
+            atomicExch(err, 1);
+            s_fail = 1;
+            for (int b = consumed; b < issued; ++b)
+                (void)mbar_wait(smem_u32(&full[b % S::kRing]), (uint32_t)((b / S::kRing) & 1));
+        }
+        umma_commit(smem_u32(&done));
+    }
+    __syncthreads();
+    if (!mbar_wait(smem_u32(&done), 0u)) {
+        atomicExch(err, 1);
+        s_fail = 1;
+    }
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (!s_fail && nblk > 0) {
+        const int row = warp * 32 + lane;   // tile row / 64 of the pair, channel row % 64
+        const int c = row & 63;
+        // every CTA adds to the same addresses: each starts at another part
+        const int parts = NP * ((nout + 15) / 16);
+#pragma unroll 1
+        for (int i = 0; i < parts; ++i) {
+            const int x = (i + (int)blockIdx.x) % parts;
+            const int q = x % NP, o0 = x / NP * 16, tap = 2 * q + (row >> 6);
+            uint32_t v[16];
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
+                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                  "=r"(v[15])
+                : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(q * 64 + o0))
+                : "memory");
+            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (o0 + j >= nout) continue;
+                const float x = __uint_as_float(v[j]);
+                if (tap < TAPS) atomicAdd(&gw[(size_t)(o0 + j) * (TAPS * 64) + tap * 64 + c], x);
+                else if (c == o0 + j) atomicAdd(&gb[c], x);   // every row of the ones holds the sums
+            }
+        }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "n"(TCOLS) : "memory");
+}
+
+template <int TAPS>
+static cudaError_t layer_dgrad_t(const __nv_bfloat16* dz, const __nv_bfloat16* wt, int wt_cols, const __nv_bfloat16* act,
+                                 __nv_bfloat16* dz_out, int frames, int M, int* err, cudaStream_t st)
+{
+    constexpr size_t smem = 1024 + (size_t)TAPS * (BM * BK * 2 + kTile);
+    static PerDevice attr;
+    if (attr.get([] {
+            return -(int)cudaFuncSetAttribute(k_dgrad<TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        }) < 0)
+        return cudaErrorInvalidConfiguration;
+    CUtensorMap mz, mw;
+    cudaError_t e;
+    if ((e = rows_map(&mz, dz, frames, M, BM))) return e;
+    if ((e = operand_map(&mw, wt, TAPS * 64, wt_cols, wt_cols, 64))) return e;
+    k_dgrad<TAPS><<<frames * (M / BM), 128, smem, st>>>(mz, mw, act, dz_out, M, err);
+    ISAR_COUNT(1);
+    return cudaGetLastError();
+}
+
+template <int TAPS>
+static cudaError_t layer_wgrad_t(const __nv_bfloat16* act, const __nv_bfloat16* dz, float* gw, float* gb, int nout,
+                                 int frames, int M, int* err, cudaStream_t st)
+{
+    static PerDevice attr;
+    if (attr.get([] {
+            return -(int)cudaFuncSetAttribute(k_wgrad<TAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                              (int)WgradSmem<TAPS>::kBytes);
+        }) < 0)
+        return cudaErrorInvalidConfiguration;
+    CUtensorMap ma, mz;
+    cudaError_t e;
+    if ((e = rows_map(&ma, act, frames, M, 64))) return e;
+    if ((e = rows_map(&mz, dz, frames, M, 64))) return e;
+    // up to 128 CTAs: a CTA's chain of row blocks costs more than the atomics
+    // of its gradient tile (16384 rows, per convolution: 32 CTAs 18.2 us, 64
+    // 14.9, 128 13.3)
+    const int nblocks = frames * (M / 64), per = (nblocks + 127) / 128;
+    k_wgrad<TAPS><<<(nblocks + per - 1) / per, 128, WgradSmem<TAPS>::kBytes, st>>>(ma, mz, gw, gb, nout, nblocks, per, M,
+                                                                                 err);
+    ISAR_COUNT(1);
+    return cudaGetLastError();
+}
+
+cudaError_t layer_dgrad(int taps, const __nv_bfloat16* dz, const __nv_bfloat16* wt, int wt_cols,
+                        const __nv_bfloat16* act, __nv_bfloat16* dz_out, int frames, int M, int* err, cudaStream_t st)
+{
+    if (frames <= 0 || M <= 0 || (M % BM) || dz == dz_out) return cudaErrorInvalidValue;
+    return taps == kTaps ? layer_dgrad_t<kTaps>(dz, wt, wt_cols, act, dz_out, frames, M, err, st)
+                         : layer_dgrad_t<1>(dz, wt, wt_cols, act, dz_out, frames, M, err, st);
+}
+
+cudaError_t layer_wgrad(int taps, const __nv_bfloat16* act, const __nv_bfloat16* dz, float* gw, float* gb, int nout,
+                        int frames, int M, int* err, cudaStream_t st)
+{
+    if (frames <= 0 || M <= 0 || (M % BM) || nout < 1 || nout > kCh) return cudaErrorInvalidValue;
+    return taps == kTaps ? layer_wgrad_t<kTaps>(act, dz, gw, gb, nout, frames, M, err, st)
+                         : layer_wgrad_t<1>(act, dz, gw, gb, nout, frames, M, err, st);
 }
 
 }  // namespace nn

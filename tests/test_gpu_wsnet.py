@@ -93,6 +93,43 @@ def test_forward_loss_and_grads_match_oracle(torch_cuda, gb300):
             assert rel < 3e-2 and cos > 0.999, (li, name, rel, cos)
 
 
+# The per-layer backward kernels (M a multiple of 128: one frame of one row
+# block, frames whose taps meet frame borders, more row blocks than CTAs) and
+# the column path (any other M), with the features' buffer overwritten between
+# the calls.  Weights are sparse multiples of 1/4 and features integers, so the
+# forward sums are exact in fp32 and round to the oracle's activations; what is
+# left is a flipped bf16 rounding of a gradient here and there: at most a few
+# of 10^4 values by 2^-8, below 1e-3 of any layer's gradient.
+@pytest.mark.parametrize("F,M", [(1, 128), (3, 128), (2, 256), (1, 1024), (70, 128), (3, 136)])
+def test_grads_match_oracle_at_row_block_edges(torch_cuda, gb300, F, M):
+    torch = torch_cuda
+    rng = np.random.default_rng(F + M)
+    parts = []
+    for r, c in wsnet.layer_shapes():
+        W = rng.choice([-0.25, 0.25], (r, c)) * (rng.random((r, c)) < (20.0 / c if r > 2 else 0.5))
+        parts += [W.ravel(), np.array([1.0, 0.0]) if r == 2 else rng.choice([0.0, 0.25], r)]
+    p = np.concatenate(parts).astype(np.float32)
+    x0 = rng.integers(-3, 4, (F, M, wsnet.CH)).astype(np.float32)
+    target = (0.3 * x0[..., 0] + rng.uniform(-0.3, 0.3, (F, M))).astype(np.float32)
+    dx = torch.from_numpy(x0).cuda().to(torch.bfloat16).contiguous()
+    dt = torch.from_numpy(target).cuda()
+    with gb300.WSNet(-(-F * M // 8) * 8, training=True) as net:
+        net.set_params(p)
+        net.forward(dx, F, M)
+        dx.fill_(float("nan"))
+        torch.cuda.synchronize()
+        loss = net.backward(dt, F, M)
+        g = net.grads()
+    want_loss, want_g = wsnet.loss_grad(p, x0, target, emulate=True)
+    assert abs(loss - want_loss) < 1e-5
+    o = 0
+    for li, (r, c) in enumerate(wsnet.layer_shapes()):
+        for name, n in (("W", r * c), ("b", r)):
+            a, w = g[o:o + n].astype(np.float64), want_g[o:o + n]
+            o += n
+            assert np.linalg.norm(a - w) / max(np.linalg.norm(w), 1e-30) < 1e-3, (li, name)
+
+
 def test_adam_steps_reduce_loss(torch_cuda, gb300):
     torch = torch_cuda
     F, M = 8, 64
