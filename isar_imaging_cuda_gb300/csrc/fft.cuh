@@ -34,6 +34,7 @@ struct FFTShape {
     static constexpr int REM = LOG % 4;
     static constexpr int NPASS = NP16 + (REM ? 1 : 0);
     static constexpr int SMEM = N + N / 16;          // float2 slots per team
+    static constexpr bool FUSE2 = REM == 1 && NP16 >= 2;   // last radix-16 and radix-2 pass in one
 };
 
 // d * exp(-+2*pi*i*j/R) with j, R compile-time after unrolling (R <= 16).
@@ -153,6 +154,41 @@ struct NoHook {
     __device__ __forceinline__ void operator()() const {}
 };
 
+// v[r] *= W_{16 NS}^{r k}, r < 16 (conjugated for INV).
+template <int N, int NS, bool INV, class Tw>
+__device__ __forceinline__ void fft_twiddle16(float2* v, int k, const Tw& tw)
+{
+    constexpr int s = N / (NS * 16);
+    if constexpr (TwTwoLevel<Tw>::value) {
+        // two-level table: look up W^k, W^2k, W^4k, W^8k and form the
+        // others as products (depth <= 3): 8 shared loads instead of 30
+        float2 w[16];
+        w[1] = tw(k * s, N);
+        w[2] = tw(2 * k * s, N);
+        w[4] = tw(4 * k * s, N);
+        w[8] = tw(8 * k * s, N);
+        w[3] = cmul(w[2], w[1]);
+        w[5] = cmul(w[4], w[1]);
+        w[6] = cmul(w[4], w[2]);
+        w[7] = cmul(w[4], w[3]);
+#pragma unroll
+        for (int r = 9; r < 16; ++r) w[r] = cmul(w[8], w[r - 8]);
+#pragma unroll
+        for (int r = 1; r < 16; ++r) {
+            float2 x = w[r];
+            if (INV) x.y = -x.y;
+            v[r] = cmul(v[r], x);
+        }
+    } else {
+#pragma unroll
+        for (int r = 1; r < 16; ++r) {
+            float2 w = tw((r * k) * s, N);
+            if (INV) w.y = -w.y;
+            v[r] = cmul(v[r], w);
+        }
+    }
+}
+
 template <int N, int R, int NS, bool INV, bool FIRST, bool LAST, class Src, class Dst, class Tw, class Hook>
 __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt, const Tw& tw, bool active,
                                          Hook& hook)
@@ -184,27 +220,8 @@ __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt,
         for (int b = 0; b < B; ++b) {
             const int j = lt + b * T;
             const int k = j & (NS - 1);
-            if constexpr (NS > 1 && R == 16 && TwTwoLevel<Tw>::value) {
-                // two-level table: look up W^k, W^2k, W^4k, W^8k and form the
-                // others as products (depth <= 3): 8 shared loads instead of 30
-                constexpr int s = N / (NS * R);
-                float2 w[16];
-                w[1] = tw(k * s, N);
-                w[2] = tw(2 * k * s, N);
-                w[4] = tw(4 * k * s, N);
-                w[8] = tw(8 * k * s, N);
-                w[3] = cmul(w[2], w[1]);
-                w[5] = cmul(w[4], w[1]);
-                w[6] = cmul(w[4], w[2]);
-                w[7] = cmul(w[4], w[3]);
-#pragma unroll
-                for (int r = 9; r < 16; ++r) w[r] = cmul(w[8], w[r - 8]);
-#pragma unroll
-                for (int r = 1; r < 16; ++r) {
-                    float2 x = w[r];
-                    if (INV) x.y = -x.y;
-                    v[b * R + r] = cmul(v[b * R + r], x);
-                }
+            if constexpr (NS > 1 && R == 16) {
+                fft_twiddle16<N, NS, INV>(&v[b * R], k, tw);
             } else if constexpr (NS > 1) {
 #pragma unroll
                 for (int r = 1; r < R; ++r) {
@@ -229,12 +246,63 @@ __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt,
     __syncthreads();
 }
 
+// The last radix-16 pass and the radix-2 pass after it (log2 N = 1 mod 4) in
+// one: the thread that holds butterfly j of the radix-16 pass needs the
+// results of butterfly j + N/32, so the two are given to lanes l and l ^ 16 of
+// a warp and half of each one's results change places by shuffles.  The
+// arithmetic is that of the two passes; a write and a read of the whole
+// transform through shared memory (the passes' bound: 512 clocks each at 8192
+// points) and two barriers are gone (with the halved shuffles of fft8192's last
+// step: hrrp 1024 x 8192 79.6 -> 73.8 us, 1024 compressed pulses 133 -> 125, 1024 x 8192
+// frame 1296 -> 1278).  Lane half h ends with the outputs
+// j + (e + 8 h) N/32 and N/2 above, e < 8, in slots 2 e and 2 e + 1.
+template <int N, bool INV, class Dst, class Tw>
+__device__ __forceinline__ void fft_last16x2(Dst& dst, float2* sm, int lt, const Tw& tw, bool active)
+{
+    constexpr int NS = N / 32;   // butterflies per half
+    static_assert(FFTShape<N>::REM == 1 && FFTShape<N>::NP16 >= 2 && FFTShape<N>::T >= 32, "transform size");
+    const int h = (lt >> 4) & 1;
+    const int jl = (lt >> 5) * 16 + (lt & 15), j = jl + h * NS;
+    float2 v[16];
+    if (active) {
+        const int pj = fpad(j);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            if constexpr ((N / 16) % 16 == 0) v[r] = sm[pj + r * (N / 16 + N / 256)];
+            else v[r] = sm[fpad(j + r * (N / 16))];
+        }
+    }
+    __syncthreads();
+    if (active) {
+        fft_twiddle16<N, NS, INV>(v, jl, tw);
+        dft_reg<16, INV>(v);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const float2 send = h ? v[e] : v[e + 8], keep = h ? v[e + 8] : v[e];
+            float2 got;
+            got.x = __shfl_xor_sync(0xffffffffu, send.x, 16);
+            got.y = __shfl_xor_sync(0xffffffffu, send.y, 16);
+            const int idx = jl + (e + 8 * h) * NS;
+            float2 w = tw(idx, N);
+            if (INV) w.y = -w.y;
+            const float2 a0 = h ? got : keep, a1 = cmul(h ? keep : got, w);
+            dst(idx, cadd(a0, a1), 2 * e);
+            dst(idx + N / 2, csub(a0, a1), 2 * e + 1);
+        }
+    }
+    __syncthreads();
+}
+
 template <int N, bool INV, int PASS, int NS, class Src, class Dst, class Tw, class Hook>
 __device__ __forceinline__ void fft_passes(Src& src, Dst& dst, float2* sm, int lt, const Tw& tw, bool active,
                                            Hook& hook)
 {
     using S = FFTShape<N>;
     constexpr int R = (PASS < S::NP16) ? 16 : (1 << S::REM);
+    if constexpr (S::FUSE2 && PASS == S::NP16 - 1) {
+        fft_last16x2<N, INV>(dst, sm, lt, tw, active);
+        return;
+    }
     fft_pass<N, R, NS, INV, PASS == 0, PASS == S::NPASS - 1>(src, dst, sm, lt, tw, active, hook);
     if constexpr (PASS + 1 < S::NPASS) fft_passes<N, INV, PASS + 1, NS * R>(src, dst, sm, lt, tw, active, hook);
 }
@@ -274,8 +342,8 @@ __device__ __forceinline__ void team_fft(Src src, Dst dst, float2* sm, int lt, c
 // a 16-point DFT over b (m0 = 2 b + a) and a radix-2 step between lanes
 // l and l ^ 16 (shuffles).  Two block barriers per transform instead of the
 // eight of the four-pass Stockham transform.
-// Output X[k0 + 16 k1 + 256 q + 4096 a] lands in register slot q of lane
-// k1 + 16 a of warp k0.
+// Output X[k0 + 16 k1 + 256 q + 4096 b] lands in register slot 2 (q mod 8) + b
+// of lane k1 + 16 (q / 8) of warp k0.
 // ---------------------------------------------------------------------------
 
 // Twiddles of row_fft<N>: the two-level table of TwShared<N>, followed at
@@ -365,16 +433,23 @@ __device__ __forceinline__ void fft8192(Src& src, Dst& dst, float2* sm, int lt, 
     const float s[16] = {0.000000000f, 0.195090322f, 0.382683432f, 0.555570233f, 0.707106781f, 0.831469612f,
                          0.923879533f, 0.980785280f, 1.000000000f, 0.980785280f, 0.923879533f, 0.831469612f,
                          0.707106781f, 0.555570233f, 0.382683432f, 0.195090322f};
+    // radix-2 step between lanes l and l ^ 16: lane half a takes q = 8 a .. 8 a + 7
+    // and half of each one's values change places
 #pragma unroll
-    for (int q = 0; q < 16; ++q) {
-        float2 o;
-        o.x = __shfl_xor_sync(0xffffffffu, v[q].x, 16);
-        o.y = __shfl_xor_sync(0xffffffffu, v[q].y, 16);
-        const float2 d0 = a ? o : v[q], d1 = a ? v[q] : o;
-        const float sn = INV ? s[q] : -s[q];   // W_32^q (forward), conj for the inverse
-        const float2 t = make_float2(d1.x * c[q] - d1.y * sn, d1.x * sn + d1.y * c[q]);
-        const float2 y = a ? csub(d0, t) : cadd(d0, t);
-        dst(w + 16 * k1 + 256 * q + 4096 * a, y, q);
+    for (int e = 0; e < 8; ++e) {
+        const float2 send = a ? v[e] : v[e + 8], keep = a ? v[e + 8] : v[e];
+        float2 got;
+        got.x = __shfl_xor_sync(0xffffffffu, send.x, 16);
+        got.y = __shfl_xor_sync(0xffffffffu, send.y, 16);
+        const float2 d0 = a ? got : keep, d1 = a ? keep : got;
+        // d1 W_32^q (forward; conj for the inverse), the fused products written
+        // out: the envelopes of the range alignment keep their rounding
+        const float cq = a ? c[e + 8] : c[e], sq = a ? s[e + 8] : s[e];
+        const float2 t = INV ? make_float2(fmaf(d1.x, cq, -(d1.y * sq)), fmaf(d1.x, sq, d1.y * cq))
+                             : make_float2(fmaf(d1.y, sq, d1.x * cq), fmaf(d1.y, cq, -(d1.x * sq)));
+        const int i = w + 16 * k1 + 256 * (e + 8 * a);
+        dst(i, cadd(d0, t), 2 * e);
+        dst(i + 4096, csub(d0, t), 2 * e + 1);
     }
 }
 
@@ -400,6 +475,8 @@ template <int N>
 __device__ __forceinline__ int fft_out_index(int lt, int slot)
 {
     using S = FFTShape<N>;
+    if constexpr (S::FUSE2)
+        return (lt >> 5) * 16 + (lt & 15) + ((slot >> 1) + 8 * ((lt >> 4) & 1)) * (N / 32) + (slot & 1) * (N / 2);
     constexpr int R = (S::NPASS - 1 < S::NP16) ? 16 : (1 << S::REM);
     const int b = slot / R, r = slot % R;
     return lt + b * S::T + r * (N / R);
@@ -410,7 +487,7 @@ __device__ __forceinline__ int row_out_index(int lt, int slot)
 {
     if constexpr (WARP && N == 8192) {
         const int lane = lt & 31;
-        return (lt >> 5) + 16 * (lane & 15) + 256 * slot + 4096 * (lane >> 4);
+        return (lt >> 5) + 16 * (lane & 15) + 256 * ((slot >> 1) + 8 * (lane >> 4)) + 4096 * (slot & 1);
     } else {
         return fft_out_index<N>(lt, slot);
     }
