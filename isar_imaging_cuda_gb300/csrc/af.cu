@@ -37,13 +37,13 @@ k_fe_stats(const float2* __restrict__ cut, int M, int rows_max, int R, float* __
     if (cmax_part != nullptr && r0 < rows_max) {
         const int r1 = min(r0 + R, rows_max);
         for (int c = tid; c < C; c += blockDim.x) {
-            float mx = 0.0f;
+            float mx = 0.0f;   // of |x|^2: the root is monotonic, and without it the loads overlap
 #pragma unroll 8
             for (int r = r0; r < r1; ++r) {
                 const float2 v = cut[(size_t)r * C + c];
-                mx = fmaxf(mx, sqrtf(v.x * v.x + v.y * v.y));
+                mx = fmaxf(mx, v.x * v.x + v.y * v.y);
             }
-            cmax_part[(size_t)blockIdx.x * C + c] = mx;
+            cmax_part[(size_t)blockIdx.x * C + c] = sqrtf(mx);
         }
     }
     const int w = tid >> 5, lane = tid & 31;

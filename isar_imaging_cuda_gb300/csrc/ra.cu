@@ -894,7 +894,7 @@ k_ra_final(const float2* x, float2* yout, const float* __restrict__ win, const i
     float acc[16];
 #pragma unroll
     for (int t = 0; t < 16; ++t) acc[t] = 0.0f;
-    float mx = 0.0f;
+    float mx2 = 0.0f;
 #pragma unroll 1
     for (int rr = 0; rr < rpc; ++rr) {
         const int row = r0 + rr;
@@ -906,11 +906,13 @@ k_ra_final(const float2* x, float2* yout, const float* __restrict__ win, const i
             if (lt == 0 && rr + 1 < rpc) st.issue(x + (size_t)(row + 1) * N, N * sizeof(float2));
         };
         const bool arp = row < arp_rows;
+        // the largest |y| through its square (the root is monotonic); the
+        // root itself only for the rows of the column sums
         auto sink = [&](int i, float2 y, int slot) {
             yr[i] = y;
-            const float a = sqrtf(y.x * y.x + y.y * y.y);
-            mx = fmaxf(mx, a);
-            if (arp) acc[slot] += a;
+            const float p = y.x * y.x + y.y * y.y;
+            mx2 = fmaxf(mx2, p);
+            if (arp) acc[slot] += sqrtf(p);
         };
         if constexpr (RAW) {
             const float invN = 1.0f / (float)N;
@@ -930,6 +932,7 @@ k_ra_final(const float2* x, float2* yout, const float* __restrict__ win, const i
 #pragma unroll
         for (int t = 0; t < 16; ++t) arp_part[(size_t)blockIdx.x * N + row_out_index<N, false>(lt, t)] = acc[t];
     }
+    float mx = sqrtf(mx2);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((lt & 31) == 0) s_red[lt >> 5] = mx;
@@ -957,30 +960,43 @@ __global__ void k_arp_reduce(const float* __restrict__ part, int nparts, int N, 
     }
 }
 
-// Standalone ARP inputs from materialised profiles y (stage entry point).
-__global__ void k_ymax(const float2* __restrict__ y, long n, unsigned* __restrict__ hmax)
+// Standalone ARP inputs from materialised profiles y (stage entry point): the
+// column sums of |y| over the first rows, in row order, by the first CTAs
+// (one thread per column, 32 loads in flight: the root's slow path keeps the
+// compiler from hoisting them), the largest |y| of all by the others.  Bound
+// by memory latency: centring and cut of 512 x 4096 profiles 88 -> 41 us (the two
+// kernels it replaces loaded one value at a time).
+constexpr int kColThreads = 64;
+__global__ void __launch_bounds__(256)
+k_yprofile(const float2* __restrict__ y, int N, int rows, long n, int col_ctas, float* __restrict__ colsum,
+           unsigned* __restrict__ hmax)
 {
-    float mx = 0.0f;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-        const float2 v = y[i];
-        mx = fmaxf(mx, sqrtf(v.x * v.x + v.y * v.y));
+    if ((int)blockIdx.x < col_ctas) {
+        if (threadIdx.x >= kColThreads) return;
+        const int c = blockIdx.x * kColThreads + threadIdx.x;
+        float s = 0.0f;
+        for (int m = 0; m < rows; m += 32) {   // rows: a multiple of 32
+            float2 v[32];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) v[q] = y[(size_t)(m + q) * N + c];
+#pragma unroll
+            for (int q = 0; q < 32; ++q) s += sqrtf(v[q].x * v[q].x + v[q].y * v[q].y);
+        }
+        colsum[c] = s;
+        return;
     }
+    // sqrt(max |y|^2): the root is monotonic
+    float mx = 0.0f;
+    const long stride = (long)(gridDim.x - col_ctas) * blockDim.x;
+#pragma unroll 8
+    for (long i = ((long)blockIdx.x - col_ctas) * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const float2 v = y[i];
+        mx = fmaxf(mx, v.x * v.x + v.y * v.y);
+    }
+    mx = sqrtf(mx);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if ((threadIdx.x & 31) == 0) atomicMax(hmax, __float_as_uint(mx));
-}
-
-__global__ void k_ycolsum(const float2* __restrict__ y, int N, int rows, float* __restrict__ colsum)
-{
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-#pragma unroll 32
-        for (int m = 0; m < rows; ++m) {
-            const float2 v = y[(size_t)m * N + n];
-            s += sqrtf(v.x * v.x + v.y * v.y);
-        }
-        colsum[n] = s;
-    }
 }
 
 // getARPMean (range_alignment.cu:524-550) for one index, float as written.
@@ -1462,9 +1478,8 @@ cudaError_t ra_run(const RAArgs& a, cudaStream_t st)
 cudaError_t arp_from_y(const float2* y, int M, int N, float* tmp, unsigned* hmax, float* arp, cudaStream_t st)
 {
     cudaMemsetAsync(hmax, 0, sizeof(unsigned), st);
-    k_ymax<<<1024, 256, 0, st>>>(y, (long)M * N, hmax);
-    ISAR_COUNT(1);
-    k_ycolsum<<<(N + 255) / 256, 256, 0, st>>>(y, N, M < 256 ? M : 256, tmp);
+    const int col_ctas = N / kColThreads;
+    k_yprofile<<<col_ctas + 4 * 152, 256, 0, st>>>(y, N, M < 256 ? M : 256, (long)M * N, col_ctas, tmp, hmax);
     ISAR_COUNT(1);
     k_arp_reduce<<<(N + 255) / 256, 256, 0, st>>>(tmp, 1, N, M, hmax, arp);
     ISAR_COUNT(1);
