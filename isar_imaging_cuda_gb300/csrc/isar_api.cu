@@ -166,7 +166,8 @@ struct isar_ctx {
     int* d_bins = nullptr;
     float2* d_sig_part = nullptr;
     float2* d_gcol = nullptr;
-    // IFDS pulse compression: spectra of the pulses in flight (grown on demand)
+    // IFDS pulse compression: the reference chirp's fixed factors and the
+    // spectra of the pulses in flight (grown on demand)
     float2* d_pc_spec = nullptr;
     size_t pc_spec_len = 0;
     unsigned* d_bar = nullptr;     // [0] autofocus grid-barrier counter, [1] its timeout flag,
@@ -959,6 +960,7 @@ ISAR_API int isar_pulse_compress(isar_ctx* c, const int16_t* d_ad, int iq_len, c
     if (S < 2 || S > nfft) return fail(ISAR_EINVAL, "reference length Fs*Tp = %d outside [2, %d]", S, nfft);
     if (pulses == 0) return ISAR_OK;
     const size_t need = (size_t)pulses * nfft;
+    const size_t base_len = ((size_t)S + 31) / 32 * 32;
     if (need > c->pc_spec_len) {
         CU(cudaStreamSynchronize(c->st));
         if (c->d_pc_spec) {
@@ -967,8 +969,10 @@ ISAR_API int isar_pulse_compress(isar_ctx* c, const int16_t* d_ad, int iq_len, c
             c->d_pc_spec = nullptr;
             c->pc_spec_len = 0;
         }
-        TRY(dalloc(c, &c->d_pc_spec, need));
+        // the chirp's fixed factors (S per context), then the spectra
+        TRY(dalloc(c, &c->d_pc_spec, base_len + need));
         c->pc_spec_len = need;
+        CU(isar::pulse_base(c->d_pc_spec, S, (float)c->r.Tp, c->st));
     }
     isar::PCArgs a{};
     a.pulses = pulses;
@@ -981,7 +985,8 @@ ISAR_API int isar_pulse_compress(isar_ctx* c, const int16_t* d_ad, int iq_len, c
     a.tp_f = (float)c->r.Tp;
     a.ad = d_ad;
     a.vel = d_velocity;
-    a.spec = c->d_pc_spec;
+    a.base = c->d_pc_spec;
+    a.spec = c->d_pc_spec + base_len;
     a.out = reinterpret_cast<float2*>(d_out);
     a.out_stride = isar::kRangeNumIfdsPc;
     a.offsets = d_offsets;

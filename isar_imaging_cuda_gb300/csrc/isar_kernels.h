@@ -189,6 +189,7 @@ struct PCArgs {
     float tp_f;              // (float)Tp
     const int16_t* ad;       // [pulses][ad_stride], I and Q interleaved
     const double* vel;       // [pulses] m/s
+    const float2* base;      // [S] chirp factors that no pulse changes (pulse_base)
     float2* spec;            // [pulses][nfft] scratch
     float2* out;             // [pulses][out_stride], 4096 cells each
     int out_stride;          // float2 per output pulse
@@ -199,6 +200,7 @@ int pc_nfft(int iq_len);
 // int16 I/Q pairs -> complex64 (samples complex values; in 8-byte and out
 // 16-byte aligned).
 cudaError_t iq16_to_c64(const int16_t* in, float* out, size_t samples, cudaStream_t st);
+cudaError_t pulse_base(float2* base, int S, float tp_f, cudaStream_t st);
 cudaError_t pulse_compress(const PCArgs& a, cudaStream_t st);
 cudaError_t ra_run(const RAArgs& a, cudaStream_t st);
 cudaError_t arp_from_y(const float2* y, int M, int N, float* tmp, unsigned* hmax, float* arp, cudaStream_t st);
