@@ -106,6 +106,26 @@ struct TwGlobal {
     __device__ __forceinline__ float2 operator()(int e, int n) const { return __ldg(&p[e * (kTwN / n)]); }
 };
 
+// W_{R NS}^{r k} of a pass: tw((r k) N / (NS R), N), from the per-pass copies
+// behind the global table where there is one.
+template <int N, int NS, int R, class Tw>
+__device__ __forceinline__ float2 tw_pass(const Tw& tw, int r, int k)
+{
+    return tw((r * k) * (N / (NS * R)), N);
+}
+template <int N, int NS, int R>
+__device__ __forceinline__ float2 tw_pass(const TwGlobal& tw, int r, int k)
+{
+    constexpr int off = NS == 16 && R == 16    ? kTwPass256
+                        : NS == 256 && R == 16 ? kTwPass4096
+                        : NS == 256 && R == 2  ? kTwPass512
+                        : NS == 256 && R == 4  ? kTwPass1024
+                        : NS == 256 && R == 8  ? kTwPass2048
+                                               : 0;
+    if constexpr (off > 0) return __ldg(&tw.p[off + r * NS + k]);
+    else return tw((r * k) * (N / (NS * R)), N);
+}
+
 // TwShared<N>: a per-CTA shared-memory table.  For N <= 2048 (or FULL) it
 // holds all N twiddles; above that (or with TWO) a two-level table
 // hi[e >> 6] * lo[e & 63] (N/64 + 64 entries, one extra complex multiply,
@@ -158,8 +178,8 @@ struct NoHook {
 template <int N, int NS, bool INV, class Tw>
 __device__ __forceinline__ void fft_twiddle16(float2* v, int k, const Tw& tw)
 {
-    constexpr int s = N / (NS * 16);
     if constexpr (TwTwoLevel<Tw>::value) {
+        constexpr int s = N / (NS * 16);
         // two-level table: look up W^k, W^2k, W^4k, W^8k and form the
         // others as products (depth <= 3): 8 shared loads instead of 30
         float2 w[16];
@@ -182,7 +202,7 @@ __device__ __forceinline__ void fft_twiddle16(float2* v, int k, const Tw& tw)
     } else {
 #pragma unroll
         for (int r = 1; r < 16; ++r) {
-            float2 w = tw((r * k) * s, N);
+            float2 w = tw_pass<N, NS, 16>(tw, r, k);
             if (INV) w.y = -w.y;
             v[r] = cmul(v[r], w);
         }
@@ -225,7 +245,7 @@ __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt,
             } else if constexpr (NS > 1) {
 #pragma unroll
                 for (int r = 1; r < R; ++r) {
-                    float2 w = tw((r * k) * (N / (NS * R)), N);
+                    float2 w = tw_pass<N, NS, R>(tw, r, k);
                     if (INV) w.y = -w.y;
                     v[b * R + r] = cmul(v[b * R + r], w);
                 }
@@ -283,7 +303,7 @@ __device__ __forceinline__ void fft_last16x2(Dst& dst, float2* sm, int lt, const
             got.x = __shfl_xor_sync(0xffffffffu, send.x, 16);
             got.y = __shfl_xor_sync(0xffffffffu, send.y, 16);
             const int idx = jl + (e + 8 * h) * NS;
-            float2 w = tw(idx, N);
+            float2 w = tw_pass<N, N / 2, 2>(tw, 1, idx);
             if (INV) w.y = -w.y;
             const float2 a0 = h ? got : keep, a1 = cmul(h ? keep : got, w);
             dst(idx, cadd(a0, a1), 2 * e);

@@ -241,11 +241,21 @@ int build_tables(isar_ctx* c)
 {
     const int M = c->M, N = c->N, C = kRangeCut;
     // twiddles exp(-2 pi i k / kTwN)
-    std::vector<float2> tw(isar::kTwN);
+    std::vector<float2> tw(isar::kTwTotal);
     for (int k = 0; k < isar::kTwN; ++k) {
         const double a = -2.0 * M_PI * (double)k / (double)isar::kTwN;
         tw[k] = make_float2((float)std::cos(a), (float)std::sin(a));
     }
+    // the passes' factors W_{R NS}^{r k} as [r][k]
+    auto pass = [&](int off, int NS, int R) {
+        for (int r = 0; r < R; ++r)
+            for (int k = 0; k < NS; ++k) tw[off + r * NS + k] = tw[r * k * (isar::kTwN / (NS * R))];
+    };
+    pass(isar::kTwPass256, 16, 16);
+    pass(isar::kTwPass4096, 256, 16);
+    pass(isar::kTwPass512, 256, 2);
+    pass(isar::kTwPass1024, 256, 4);
+    pass(isar::kTwPass2048, 256, 8);
     CU(cudaMemcpyAsync(c->d_tw, tw.data(), tw.size() * sizeof(float2), cudaMemcpyHostToDevice, c->st));
     // range-alignment window: hamming(n) * cos(pi * n) (range_alignment.cu:195-201)
     std::vector<float> ham(N), win(N);
@@ -341,7 +351,7 @@ int create_impl(isar_ctx* c)
     TRY(dalloc(c, &c->d_post, (size_t)M * C));
     TRY(dalloc(c, &c->d_V, (size_t)C * 2 * M));
     TRY(dalloc(c, &c->d_hamM, M));
-    TRY(dalloc(c, &c->d_tw, isar::kTwN));
+    TRY(dalloc(c, &c->d_tw, isar::kTwTotal));
     CU(cudaMemsetAsync(c->d_dec, 0, 16 * sizeof(int), c->st));
     CU(cudaMemsetAsync(c->d_fdec, 0, 16 * sizeof(int), c->st));
     return build_tables(c);

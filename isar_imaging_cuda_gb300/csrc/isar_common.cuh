@@ -16,6 +16,17 @@ constexpr int kEntropyIters = 120;      // FAST_ENTROPY_ITERATION_NUM
 constexpr int kMaxN = 8192;            // largest supported range_num
 constexpr int kMaxM = 1024;             // largest supported echo_num
 constexpr int kTwN = 16384;             // twiddle table length
+// The table is followed by the factors W_{R NS}^{r k} of the transforms' passes
+// as [r][k] (k < NS), so that neighbouring lanes (neighbouring k) read
+// neighbouring entries: in the table itself they lie r kTwN / (R NS) apart, a
+// gather of up to 32 lines per load that held the row transforms up (hrrp
+// 1024 x 8192 73 -> 37 us, 512 x 4096 IFDS frame 1175 -> 1155).  Offsets of (NS, R):
+constexpr int kTwPass256 = kTwN;                  // (16, 16)
+constexpr int kTwPass4096 = kTwPass256 + 256;     // (256, 16)
+constexpr int kTwPass512 = kTwPass4096 + 4096;    // (256, 2)
+constexpr int kTwPass1024 = kTwPass512 + 512;     // (256, 4)
+constexpr int kTwPass2048 = kTwPass1024 + 1024;   // (256, 8)
+constexpr int kTwTotal = kTwPass2048 + 2048;
 
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {

@@ -1287,7 +1287,7 @@ __global__ void __launch_bounds__(N / 16) k_fft_rows(float2* x, const float2* __
 // rows are swapped, transformed and swapped again.  Both swaps are folded
 // into the transform's load and store indices.
 template <int N>
-__global__ void __launch_bounds__(N / 16)
+__global__ void __launch_bounds__(N / 16, 1024 / (N / 16))
 k_hrrp(const float2* x, float2* out, const float* __restrict__ ham, int ifds, const float2* __restrict__ tw)
 {
     extern __shared__ float4 dyn_smem[];
