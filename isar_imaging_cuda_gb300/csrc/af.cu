@@ -7,6 +7,7 @@
 
 #include "fft.cuh"
 #include "isar_kernels.h"
+#include "launch.cuh"
 #include "nn.h"
 
 namespace isar {
@@ -32,6 +33,7 @@ __global__ void __launch_bounds__(256)
 k_fe_stats(const float2* __restrict__ cut, int M, int rows_max, int R, float* __restrict__ cmax_part,
            float2* __restrict__ dsum)
 {
+    pdl_begin();
     const int r0 = blockIdx.x * R;
     const int tid = threadIdx.x;
     if (cmax_part != nullptr && r0 < rows_max) {
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(256)
 k_af_doppler(const float2* __restrict__ cut, const int* __restrict__ bins, const int* __restrict__ fdec,
              int M, float2* __restrict__ dsum)
 {
+    pdl_begin();
     const int U = fdec[1];
     const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int m = w;
@@ -109,6 +112,7 @@ k_fe_phase(const float* __restrict__ cmax_part, int nparts, const float2* __rest
     __shared__ unsigned s_nan[32];
     __shared__ int s_cnt[32];
     __shared__ int s_sum[32];
+    pdl_begin();
     const int tid = threadIdx.x;
     const int lane = tid & 31, w = tid >> 5, nw = blockDim.x >> 5;
     // inclusive scan of arg(s); a NaN reaches every later phase
@@ -226,6 +230,7 @@ k_fe_colfft(const float2* __restrict__ cut, const float2* __restrict__ phase, do
     const int c0 = blockIdx.x * CB;
     float2* twt = smb + CB * F::SMEM;
     TwShared<M>::fill(twt, tw, tid, blockDim.x);
+    pdl_begin();
     for (int i = tid; i < M * CB; i += blockDim.x) {
         const int m = i / CB, cc = i % CB;
         smb[cc * F::SMEM + fpad(m)] = cmul(phase[m], cut[(size_t)m * C + c0 + cc]);
@@ -316,6 +321,7 @@ k_fe_select(const double* __restrict__ E, const double* __restrict__ H, int* __r
     __shared__ SelKey sm[C];
     __shared__ int s_flag[C];
     __shared__ int s_cnt[C / 32];
+    pdl_begin();
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int tgt = fdec[0], U = fdec[1];
     SelKey v;
@@ -745,6 +751,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     for (int i = tid; i < M; i += A::THREADS) T1[i] = tw[(i / L) * (i & (L - 1)) * (kTwN / M)];
     for (int i = tid; i < P * Q; i += A::THREADS) T2[i] = tw[(i / Q) * (i & (Q - 1)) * (kTwN / L)];
     float2* ta = tiles + slot * A::TILE;
+    pdl_begin();
     const int U = f.fdec[1];
     if (U > f.max_u) return;   // the whole cluster, before any message
     const int bpc = (U + CL - 1) / CL;
@@ -1072,6 +1079,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
 // cut[m][c] *= phase[m]  (phase_adjustment.cu:324)
 __global__ void k_af_apply(float2* __restrict__ cut, const float2* __restrict__ phase, int M)
 {
+    pdl_begin();
     const int m = blockIdx.x;
     const float2 p = phase[m];
     for (int c = threadIdx.x; c < C; c += blockDim.x) cut[(size_t)m * C + c] = cmul(p, cut[(size_t)m * C + c]);
@@ -1104,9 +1112,10 @@ static AfKernel af_kernel(int cl)
     return cl == 16 ? k_af_cluster<M, 16> : cl == 8 ? k_af_cluster<M, 8> : k_af_cluster<M, 4>;
 }
 
-// The launch of one cluster of cl CTAs (`at` must outlive the configuration).
+// The launch of one cluster of cl CTAs (the two attributes `at` must outlive
+// the configuration).
 template <int M>
-static cudaLaunchConfig_t af_cluster_config(int cl, cudaStream_t st, cudaLaunchAttribute* at)
+static cudaLaunchConfig_t af_cluster_config(int cl, bool overlap, cudaStream_t st, cudaLaunchAttribute* at)
 {
     cudaLaunchConfig_t cfg = {};
     at->id = cudaLaunchAttributeClusterDimension;
@@ -1117,8 +1126,10 @@ static cudaLaunchConfig_t af_cluster_config(int cl, cudaStream_t st, cudaLaunchA
     cfg.blockDim = dim3(AFC<M>::THREADS);
     cfg.dynamicSmemBytes = AFC<M>::SMEM;
     cfg.stream = st;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = overlap ? 2 : 1;
     return cfg;
 }
 
@@ -1136,8 +1147,8 @@ static int af_cluster_probe()
             return -(int)e;
         if (cl > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1))
             (void)cudaGetLastError();
-        cudaLaunchAttribute at;
-        const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, nullptr, &at);
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, false, nullptr, at);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n > 0 && best == 0) best = cl;
         (void)cudaGetLastError();
@@ -1159,8 +1170,8 @@ static cudaError_t af_cluster_launch(const FEArgs& a, int cl, int max_u, cudaStr
     if (mx < 0) return (cudaError_t)(-mx);
     if (cl != 4 && cl != 8 && cl != 16) return cudaErrorInvalidValue;
     if (cl > mx) return cudaErrorInvalidClusterSize;
-    cudaLaunchAttribute at;
-    const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, st, &at);
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, a.overlap != 0, st, at);
     AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol, a.bar + 3, max_u};
     cudaError_t e = cudaLaunchKernelEx(&cfg, af_kernel<M>(cl), fr, a.iters, a.tol, a.tw);
     if (e == cudaSuccess) ISAR_COUNT(1);
@@ -1210,23 +1221,21 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
     const int rows_max = M < 256 ? M : 256;
     const int R = 8;
     const int nparts = (rows_max + R - 1) / R;
-    k_fe_stats<<<(M + R - 1) / R, 256, 0, st>>>(a.cut, M, rows_max, R, a.cmax_part, a.dsum);
-    ISAR_COUNT(1);
-    k_fe_phase<<<M / 32, M, 0, st>>>(a.cmax_part, nparts, a.dsum, M, a.phase, a.fdec);
-    ISAR_COUNT(1);
-    k_fe_colfft<M, CB><<<C / CB, CB * F::T, smem, st>>>(a.cut, a.phase, a.E, a.H, a.tw);
-    ISAR_COUNT(1);
-    k_fe_select<<<1, C, 0, st>>>(a.E, a.H, a.fdec, a.bins);
-    ISAR_COUNT(1);
-    k_af_doppler<<<(M * 32 + 255) / 256, 256, 0, st>>>(a.cut, a.bins, a.fdec, M, a.dsum);
-    ISAR_COUNT(1);
-    k_fe_phase<<<M / 32, M, 0, st>>>(nullptr, 0, a.dsum, M, a.phase, a.fdec);
-    ISAR_COUNT(1);
+    cudaError_t e;
+    if ((e = launch_after(a.overlap == 1, k_fe_stats, (M + R - 1) / R, 256, 0, st, a.cut, M, rows_max, R, a.cmax_part, a.dsum)))
+        return e;
+    if ((e = launch_after(a.overlap, k_fe_phase, M / 32, M, 0, st, a.cmax_part, nparts, a.dsum, M, a.phase, a.fdec)))
+        return e;
+    if ((e = launch_after(a.overlap, k_fe_colfft<M, CB>, C / CB, CB * F::T, smem, st, a.cut, a.phase, a.E, a.H, a.tw)))
+        return e;
+    if ((e = launch_after(a.overlap, k_fe_select, 1, C, 0, st, a.E, a.H, a.fdec, a.bins))) return e;
+    if ((e = launch_after(a.overlap, k_af_doppler, (M * 32 + 255) / 256, 256, 0, st, a.cut, a.bins, a.fdec, M, a.dsum)))
+        return e;
+    if ((e = launch_after(a.overlap, k_fe_phase, M / 32, M, 0, st, nullptr, 0, a.dsum, M, a.phase, a.fdec))) return e;
     if (a.pre_only) return cudaGetLastError();
     if (a.ws_w && (a.af_cluster == 0 || a.iters == 0)) return cudaErrorInvalidValue;
     if (a.ws_w) {
         // learned warm start: features -> network -> second start phase
-        cudaError_t e;
         if ((e = nn::features(a.cut, a.E, a.dsum, M, a.ws_a->act[0], a.ws_psi, st))) return e;
         if ((e = nn::forward(*a.ws_w, *a.ws_a, 1, M, a.ws_err, st))) return e;
         if ((e = nn::ws_phase(a.ws_psi, a.ws_a->out, M, a.ws_phase, st))) return e;
@@ -1245,11 +1254,9 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
     const int cl = auto16 ? 16 : a.af_cluster;
     const int max_u = auto16 && M == 512 ? 256 : C;
     if (a.iters > 0 && cl > 0) {
-        cudaError_t e = af_cluster_launch<M>(a, cl, max_u, st);
-        if (e) return e;
+        if ((e = af_cluster_launch<M>(a, cl, max_u, st))) return e;
     }
     if (a.iters > 0 && (cl == 0 || max_u < C)) {
-        cudaError_t e;
         if ((e = cudaMemsetAsync(a.bar, 0, 2 * sizeof(unsigned), st))) return e;
         int min_u = cl == 0 ? 0 : max_u + 1;
         const float2* cut = a.cut;
@@ -1270,12 +1277,12 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
         ISAR_COUNT(1);
     }
     if (a.defer_apply) return cudaGetLastError();   // the imaging applies the phase(s)
-    if (a.ws_w && a.iters > 0 && a.af_cluster > 0)
+    if (a.ws_w && a.iters > 0 && a.af_cluster > 0) {
         k_af_apply2<<<M, 256, 0, st>>>(a.cut, a.phase, a.ws_phase, a.cut2, M);
-    else
-        k_af_apply<<<M, 256, 0, st>>>(a.cut, a.phase, M);
-    ISAR_COUNT(1);
-    return cudaGetLastError();
+        ISAR_COUNT(1);
+        return cudaGetLastError();
+    }
+    return launch_after(a.overlap, k_af_apply, M, 256, 0, st, a.cut, a.phase, M);
 }
 
 cudaError_t fe_run(const FEArgs& a, cudaStream_t st)

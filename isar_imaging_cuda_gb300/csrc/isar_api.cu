@@ -195,6 +195,8 @@ struct isar_ctx {
     int af_iters = isar::kEntropyIters;
     // cached CUDA graphs of whole frames
     bool use_graphs = true;
+    bool overlap = true;           // kernels overlap their predecessors' ends (launch.cuh)
+    bool reset_node = false;       // RAArgs::reset_node
     std::vector<CachedGraph> graphs;
     unsigned long long graph_tick = 0;
     // learned warm start: the attached network and this context's
@@ -209,6 +211,12 @@ struct isar_ctx {
     int* d_ws_err = nullptr;
     bool ws_alloc = false;
 };
+
+void isar::set_lane(isar_ctx* c, bool reset_node)
+{
+    c->overlap = false;
+    c->reset_node = reset_node;
+}
 
 namespace {
 
@@ -381,6 +389,8 @@ isar::RAArgs ra_args(isar_ctx* c, const float2* x, float2* y, bool hpc, bool hrr
     a.rpc_final = c->ra_rpc_final;
     a.given_shifts = c->ra_given ? 1 : 0;
     a.err = c->d_bar + 2;
+    a.overlap = c->overlap;
+    a.reset_node = c->reset_node;
     return a;
 }
 
@@ -405,6 +415,7 @@ isar::FEArgs fe_args(isar_ctx* c, float2* cut, int iters)
     a.af_cluster = c->af_cluster;
     a.tol = c->af_tol;
     a.af_stat = c->d_fdec + 4;
+    a.overlap = c->overlap;
     if (c->ws_w) {
         a.ws_w = c->ws_w;
         a.ws_a = &c->ws_a;
@@ -431,6 +442,7 @@ isar::PostArgs post_args(isar_ctx* c, float2* cut, int flags, float* img)
     a.hamM = c->d_hamM;
     a.img = img;
     a.tw = c->d_tw;
+    a.overlap = c->overlap;
     return a;
 }
 
@@ -471,7 +483,7 @@ int run_frame_eager(isar_ctx* c, const float2* x, const double* d_vel, int flags
         flags &= ~ISAR_FLAG_IQ16;
     }
     TRY(run_range_align(c, x, c->d_x, d_vel, flags));
-    CU(isar::center_cut(c->d_arp, c->d_x, c->M, c->N, c->d_dec, c->d_cut, c->st));
+    CU(isar::center_cut(c->d_arp, c->d_x, c->M, c->N, c->d_dec, c->d_cut, c->st, c->overlap));
     // With MTRC at 512 pulses or more the imaging applies the autofocus
     // phase itself (in the CZT's load), so the cut stays unphased and the
     // rows' transform of the MTRC is shared by both legs of a warm start.
@@ -914,7 +926,7 @@ ISAR_API int isar_stage_center_cut(isar_ctx* c, const float* d_y, float* d_cut)
     if (!d_y || !d_cut) return fail(ISAR_EINVAL, "null argument");
     const float2* y = reinterpret_cast<const float2*>(d_y);
     CU(isar::arp_from_y(y, c->M, c->N, c->d_part, c->d_hmax, c->d_arp, c->st));
-    CU(isar::center_cut(c->d_arp, y, c->M, c->N, c->d_dec, reinterpret_cast<float2*>(d_cut), c->st));
+    CU(isar::center_cut(c->d_arp, y, c->M, c->N, c->d_dec, reinterpret_cast<float2*>(d_cut), c->st, true));
     return ISAR_OK;
 }
 
@@ -926,6 +938,7 @@ ISAR_API int isar_stage_fast_entropy(isar_ctx* c, float* d_cut, int iterations)
     // final images, which only the whole frame produces
     isar::FEArgs a = fe_args(c, reinterpret_cast<float2*>(d_cut), iterations);
     a.ws_w = nullptr;
+    a.overlap = 2;   // the first kernel waits for all of the caller's work
     CU(isar::fe_run(a, c->st));
     return ISAR_OK;
 }
@@ -934,7 +947,9 @@ ISAR_API int isar_stage_post(isar_ctx* c, float* d_cut, int flags, float* d_img)
 {
     TRY(check_ctx(c));
     if (!d_cut || !d_img) return fail(ISAR_EINVAL, "null argument");
-    CU(isar::post_run(post_args(c, reinterpret_cast<float2*>(d_cut), flags, d_img), c->st));
+    isar::PostArgs pa = post_args(c, reinterpret_cast<float2*>(d_cut), flags, d_img);
+    pa.overlap = 2;   // the first kernel waits for all of the caller's work
+    CU(isar::post_run(pa, c->st));
     return ISAR_OK;
 }
 

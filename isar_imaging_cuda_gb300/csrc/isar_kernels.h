@@ -7,6 +7,8 @@
 #include <atomic>
 #include <mutex>
 
+struct isar_ctx;   // an imaging context (isar_api.cu)
+
 namespace isar {
 
 namespace nn {
@@ -81,6 +83,8 @@ struct RAArgs {
     int given_shifts;        // use the shifts already in `shifts` (test hook)
     unsigned* err;           // set when a row-copy wait runs out (rows invalid)
     int x_iq16;              // x holds int16 I/Q pairs (level 0 reads them directly)
+    int overlap;             // kernels overlap their predecessors' ends (launch.cuh)
+    int reset_node;          // the profile maximum is reset by a memset of its own (isar_batch.cpp)
 };
 
 // Poll limit of the autofocus grid barrier (about a second of polling), and
@@ -131,6 +135,8 @@ struct FEArgs {
     float2* cut2;            // [M][512] the learned leg's phase applied to the cut (warm start;
                              // not written with defer_apply, where the imaging applies it)
     int* ws_err;             // GEMM wait-timeout flag
+    int overlap;             // kernels overlap their predecessors' ends (launch.cuh): 1 all,
+                             // 2 all but the first
     int pre_only;            // stop after the bin selection and the Doppler start phase
     int defer_apply;         // leave the cut unphased: the imaging applies the phase(s)
                              // (PostArgs::phase; MTRC at M >= 512 only)
@@ -168,6 +174,7 @@ struct PostArgs {
     // holds the rows' transform of this cut (the second leg of a frame).
     const float2* phase;
     int rows_ready;
+    int overlap;             // as FEArgs::overlap
 };
 
 cudaError_t hpc_coef(const double* vel, int M, double coef_over_fs2, int64_t* hq, cudaStream_t st);
@@ -204,7 +211,11 @@ cudaError_t pulse_base(float2* base, int S, float tp_f, cudaStream_t st);
 cudaError_t pulse_compress(const PCArgs& a, cudaStream_t st);
 cudaError_t ra_run(const RAArgs& a, cudaStream_t st);
 cudaError_t arp_from_y(const float2* y, int M, int N, float* tmp, unsigned* hmax, float* arp, cudaStream_t st);
-cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec, float2* cut, cudaStream_t st);
+cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec, float2* cut, cudaStream_t st,
+                       bool overlap = false);
+// Makes the context a batch's lane: its kernels do not overlap their
+// predecessors' ends (launch.cuh), and RAArgs::reset_node is set as given.
+void set_lane(isar_ctx* c, bool reset_node);
 // Raises k_center's dynamic shared-memory limit to the kMaxN case on the
 // calling thread's current device (the attribute is per device).
 cudaError_t center_prepare_current_device();

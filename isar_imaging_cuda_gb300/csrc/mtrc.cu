@@ -5,6 +5,7 @@
 
 #include "fft.cuh"
 #include "isar_kernels.h"
+#include "launch.cuh"
 
 namespace isar {
 
@@ -17,6 +18,7 @@ __global__ void __launch_bounds__(256) k_mtrc_rows(const float2* __restrict__ cu
 {
     using F = FFTShape<C>;
     __shared__ float2 smb[8 * F::SMEM];
+    pdl_begin();
     const int team = threadIdx.x / F::T, lt = threadIdx.x % F::T;
     const int m = blockIdx.x * 8 + team;
     const float2* xr = cut + (size_t)m * C;
@@ -56,6 +58,7 @@ k_czt(const float2* __restrict__ st, const float2* __restrict__ pre, const float
     float2* tile = smb + CB * F::SMEM;   // [M][CB]
     const int tid = threadIdx.x;
     const int team = tid / F::T, lt = tid % F::T;
+    pdl_begin();
     const int c0 = blockIdx.x * CB;
     for (int i = tid; i < M * CB; i += blockDim.x) {
         const int k = i / CB, cc = i % CB;
@@ -133,6 +136,7 @@ k_mtrc_cols(const float2* __restrict__ in, float2* __restrict__ out, const float
     float2* smb = reinterpret_cast<float2*>(dyn_smem);
     const int tid = threadIdx.x;
     const int team = tid / F::T, lt = tid % F::T;
+    pdl_begin();
     const int c0 = blockIdx.x * CB;
     for (int i = tid; i < M * CB; i += blockDim.x) {
         const int m = i / CB, cc = i % CB;
@@ -157,6 +161,7 @@ __global__ void __launch_bounds__(256) k_mtrc_rowfft(const float2* __restrict__ 
 {
     using F = FFTShape<C>;
     __shared__ float2 smb[8 * F::SMEM];
+    pdl_begin();
     const int team = threadIdx.x / F::T, lt = threadIdx.x % F::T;
     const int m = blockIdx.x * 8 + team;
     const float2* xr = in + (size_t)m * C;
@@ -177,6 +182,7 @@ __global__ void __launch_bounds__(256) k_mtrc_rowfft_abs(const float2* __restric
 {
     using F = FFTShape<C>;
     __shared__ float2 smb[8 * F::SMEM];
+    pdl_begin();
     const int team = threadIdx.x / F::T, lt = threadIdx.x % F::T;
     const int m = blockIdx.x * 8 + team;
     const float2* xr = in + (size_t)m * C;
@@ -206,6 +212,7 @@ k_post(const float2* __restrict__ cut, int src_shift, const float* __restrict__ 
     float* tile = reinterpret_cast<float*>(smb + CB * F::SMEM);   // [M][CB]
     const int tid = threadIdx.x;
     const int team = tid / F::T, lt = tid % F::T;
+    pdl_begin();
     const int c0 = blockIdx.x * CB;
     for (int i = tid; i < M * CB; i += blockDim.x) {
         const int m = i / CB, cc = i % CB;
@@ -263,35 +270,35 @@ static cudaError_t post_run_m(const PostArgs& a, cudaStream_t st)
     int src_shift = 0;
     const float2* src = a.cut;
     if ((a.phase || a.rows_ready) && !(a.mtrc && M >= 512)) return cudaErrorInvalidValue;
+    cudaError_t e;
+    bool over = a.overlap == 1;   // 2: from the second kernel on
     if (a.mtrc) {
         if (!a.rows_ready) {
-            if (a.data_type == 1) k_mtrc_rows<false><<<M / 8, 256, 0, st>>>(a.cut, a.st, a.tw);
-            else k_mtrc_rows<true><<<M / 8, 256, 0, st>>>(a.cut, a.st, a.tw);
-            ISAR_COUNT(1);
+            if ((e = launch_after(over, a.data_type == 1 ? k_mtrc_rows<false> : k_mtrc_rows<true>, M / 8, 256, 0, st, a.cut,
+                                  a.st, a.tw)))
+                return e;
+            over = a.overlap != 0;
         }
         if constexpr (M >= 512) {
             // the column IFFT, window and column FFT as one column correction
             // (see k_czt, COLMEAN), then the rows form the image; st is only
             // read from here on, so a second leg reuses it (rows_ready)
-            k_czt<M, CZ, true><<<C / CZ, CZ * FL::T, smem_czt, st>>>(a.st, a.pre, a.post, a.V, a.st2, a.tw,
-                                                                      a.hamM, a.data_type == 1, a.phase);
-            ISAR_COUNT(1);
-            k_mtrc_rowfft_abs<<<M / 8, 256, 0, st>>>(a.st2, a.img, a.data_type == 1, a.tw);
-            ISAR_COUNT(1);
-            return cudaGetLastError();
+            if ((e = launch_after(over, k_czt<M, CZ, true>, C / CZ, CZ * FL::T, smem_czt, st, a.st, a.pre, a.post, a.V, a.st2,
+                                  a.tw, a.hamM, a.data_type == 1, a.phase)))
+                return e;
+            return launch_after(a.overlap != 0, k_mtrc_rowfft_abs, M / 8, 256, 0, st, a.st2, a.img, a.data_type == 1, a.tw);
         }
-        k_czt<M, CZ><<<C / CZ, CZ * FL::T, smem_czt, st>>>(a.st, a.pre, a.post, a.V, a.st2, a.tw);
-        ISAR_COUNT(1);
-        k_mtrc_cols<M, CB><<<C / CB, CB * F::T, smem_cols, st>>>(a.st2, a.st, a.tw);
-        ISAR_COUNT(1);
-        k_mtrc_rowfft<<<M / 8, 256, 0, st>>>(a.st, a.st2, a.data_type == 1, a.tw);
-        ISAR_COUNT(1);
+        if ((e = launch_after(over, k_czt<M, CZ, false>, C / CZ, CZ * FL::T, smem_czt, st, a.st, a.pre, a.post, a.V, a.st2,
+                              a.tw, nullptr, 0, nullptr)))
+            return e;
+        over = a.overlap != 0;
+        if ((e = launch_after(over, k_mtrc_cols<M, CB>, C / CB, CB * F::T, smem_cols, st, a.st2, a.st, a.tw))) return e;
+        if ((e = launch_after(over, k_mtrc_rowfft, M / 8, 256, 0, st, a.st, a.st2, a.data_type == 1, a.tw))) return e;
         src = a.st2;
         src_shift = M / 2;   // final column fftshift of mtrc (mtrc.cu:69)
     }
-    k_post<M, CB><<<C / CB, CB * F::T, smem_post, st>>>(src, src_shift, a.hamM, a.data_type == 1, a.img, a.tw);
-    ISAR_COUNT(1);
-    return cudaGetLastError();
+    return launch_after(over, k_post<M, CB>, C / CB, CB * F::T, smem_post, st, src, src_shift, a.hamM, a.data_type == 1, a.img,
+                        a.tw);
 }
 
 cudaError_t post_run(const PostArgs& a, cudaStream_t st)

@@ -29,6 +29,7 @@
 #include "cells_fixed.h"
 #include "fft.cuh"
 #include "isar_kernels.h"
+#include "launch.cuh"
 
 namespace isar {
 
@@ -182,10 +183,11 @@ __global__ void k_hpc_coef(const double* __restrict__ vel, int M, double coef_ov
     }
 }
 
-// S[m] = 0 and its fixed-point phase slope SQ[m] = 0.
-__global__ void k_zero_shift(double* __restrict__ S, int64_t* __restrict__ SQ, int n)
+// S[m] = 0 and its fixed-point phase slope SQ[m] = 0; the profile maximum too.
+__global__ void k_zero_shift(double* __restrict__ S, int64_t* __restrict__ SQ, int n, unsigned* __restrict__ hmax)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *hmax = 0;
     if (i < n) {
         S[i] = 0.0;
         SQ[i] = 0;
@@ -725,6 +727,7 @@ k_ra_spec0(const float2* x, float2* xw, const float* __restrict__ win, const int
         sb.issue(src + (size_t)(2 * j + 1) * kRowBytes, kRowBytes);
     }
     RaTw<N>::fill(twt, tw, lt, F::T);
+    pdl_begin();   // the echoes copied above are older than the kernel before
     __syncthreads();
     const RaTw<N> tws{twt};
     const float invN = 1.0f / (float)N;
@@ -824,8 +827,9 @@ k_ra_spec(const float2* __restrict__ wprev, float2* __restrict__ wout, double* _
     // the shifts of the second group's rows: read here, where the load's
     // latency is hidden, written at the end
     const size_t row2 = (size_t)(2 * j + 1) * s + lt;
-    const double s_old = lt < s ? S[row2] : 0.0;
     RaTw<N>::fill(twt, tw, lt, F::T);
+    pdl_begin();
+    const double s_old = lt < s ? S[row2] : 0.0;
     __syncthreads();
     const RaTw<N> tws{twt};
     const float2* wa = wprev + (size_t)2 * j * N;
@@ -884,11 +888,12 @@ k_ra_final(const float2* x, float2* yout, const float* __restrict__ win, const i
     const int r0 = blockIdx.x * rpc;
     float2* twt = sm + F::SMEM;
     RowStage st{twt + RaTw<N>::kEntries, &bar, err, 0u};
+    RaTw<N>::fill(twt, tw, lt, F::T);
+    pdl_begin();
     if (lt == 0) {
         st.init();
         st.issue(x + (size_t)r0 * N, N * sizeof(float2));
     }
-    RaTw<N>::fill(twt, tw, lt, F::T);
     __syncthreads();
     const RaTw<N> tws{twt};
     float acc[16];
@@ -948,6 +953,7 @@ k_ra_final(const float2* x, float2* yout, const float* __restrict__ win, const i
 __global__ void k_arp_reduce(const float* __restrict__ part, int nparts, int N, int M,
                              const unsigned* __restrict__ hmax, float* __restrict__ arp)
 {
+    pdl_begin();
     // an all-zero frame (max 0) gives a zero profile rather than 0/0
     const float hm = __uint_as_float(*hmax);
     const float inv = hm > 0.0f ? 1.0f / hm : 0.0f;
@@ -1143,6 +1149,7 @@ k_center(const float* __restrict__ arp_g, const float2* __restrict__ y, int N, i
     __shared__ int2 red_n[32];
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int T = N / 8;
+    pdl_begin();
     // the profile, 8 consecutive cells per thread, and |Re| + |Im| of row 0
     // (for the cut below: its load overlaps the sort)
     unsigned k[8];
@@ -1251,6 +1258,7 @@ k_center(const float* __restrict__ arp_g, const float2* __restrict__ y, int N, i
 // cut[m][c] = centred y[m][off + c] = y[m][(off + c - shift) mod N]
 __global__ void k_cut(const float2* __restrict__ y, int N, const int* __restrict__ dec, float2* __restrict__ cut)
 {
+    pdl_begin();
     const int m = blockIdx.x;
     const int shift = dec[1], off = dec[2];
     for (int c = threadIdx.x; c < kRangeCut; c += blockDim.x)
@@ -1371,7 +1379,7 @@ static cudaError_t ra_run_n(const RAArgs& a, cudaStream_t st)
     const int T = N / 16;
     int L = 0;
     while ((1 << L) < M) ++L;
-    k_zero_shift<<<(M + 255) / 256, 256, 0, st>>>(a.S, a.SQ, M);
+    k_zero_shift<<<(M + 255) / 256, 256, 0, st>>>(a.S, a.SQ, M, a.hmax);
     ISAR_COUNT(1);
     // spectral envelope merge: merged group spectra ping-pong between env_a
     // (M/2 x N complex) and part (M/4 x N complex)
@@ -1379,19 +1387,16 @@ static cudaError_t ra_run_n(const RAArgs& a, cudaStream_t st)
     if (spectral) {
         float2* wb[2] = {reinterpret_cast<float2*>(a.env_a), reinterpret_cast<float2*>(a.part)};
         float2* w0 = L > 1 ? wb[0] : nullptr;
-        if (a.x_iq16)
-            k_ra_spec0<N, true><<<M / 2, T, spec0_smem<N>(), st>>>(a.x, a.y, a.win, a.hq, a.S, a.SQ, w0, a.shifts,
-                                                                   a.given_shifts, a.tw, a.err);
-        else
-            k_ra_spec0<N, false><<<M / 2, T, spec0_smem<N>(), st>>>(a.x, a.y, a.win, a.hq, a.S, a.SQ, w0, a.shifts,
-                                                                    a.given_shifts, a.tw, a.err);
-        ISAR_COUNT(1);
+        if ((e = launch_after(a.overlap, a.x_iq16 ? k_ra_spec0<N, true> : k_ra_spec0<N, false>, M / 2, T, spec0_smem<N>(),
+                              st, a.x, a.y, a.win, a.hq, a.S, a.SQ, w0, a.shifts, a.given_shifts, a.tw, a.err)))
+            return e;
         int off = M / 2;
         for (int lv = 1; lv < L; ++lv) {
             const int pairs = M >> (lv + 1);
-            k_ra_spec<N><<<pairs, T, corr_smem<N>(), st>>>(wb[(lv - 1) & 1], lv == L - 1 ? nullptr : wb[lv & 1], a.S,
-                                                          a.SQ, lv, a.shifts + off, a.given_shifts, a.tw);
-            ISAR_COUNT(1);
+            if ((e = launch_after(a.overlap, k_ra_spec<N>, pairs, T, corr_smem<N>(), st, wb[(lv - 1) & 1],
+                                  lv == L - 1 ? nullptr : wb[lv & 1], a.S, a.SQ, lv, a.shifts + off, a.given_shifts,
+                                  a.tw)))
+                return e;
             off += pairs;
         }
         if ((e = cudaGetLastError())) return e;
@@ -1444,22 +1449,18 @@ static cudaError_t ra_run_n(const RAArgs& a, cudaStream_t st)
         shift_off += pairs;
         if ((e = cudaGetLastError())) return e;
     }
+    if (a.reset_node && (e = cudaMemsetAsync(a.hmax, 0, sizeof(unsigned), st))) return e;
     // final IFFT + ARP partials + hmax
-    cudaMemsetAsync(a.hmax, 0, sizeof(unsigned), st);
     const int arp_rows = M < 256 ? M : 256;
     int rpcf = a.rpc_final;
     while (rpcf > 1 && (M % rpcf)) rpcf >>= 1;
     if (L == 0 && a.x_iq16) return cudaErrorInvalidValue;   // a single pulse: no level reads x
-    if (L == 0)
-        k_ra_final<N, true><<<M / rpcf, T, ra_fft_smem<N>(), st>>>(a.x, a.y, a.win, a.hq, a.SQ, rpcf, arp_rows, a.part,
-                                                                  a.hmax, a.tw, a.err);
-    else
-        k_ra_final<N, false><<<M / rpcf, T, ra_fft_smem<N>(), st>>>(a.y, a.y, a.win, a.hq, a.SQ, rpcf, arp_rows,
-                                                                   a.part, a.hmax, a.tw, a.err);
-    ISAR_COUNT(1);
+    if ((e = launch_after(a.overlap, L == 0 ? k_ra_final<N, true> : k_ra_final<N, false>, M / rpcf, T, ra_fft_smem<N>(), st,
+                          L == 0 ? a.x : a.y, a.y, a.win, a.hq, a.SQ, rpcf, arp_rows, a.part, a.hmax, a.tw, a.err)))
+        return e;
     const int nparts = (arp_rows + rpcf - 1) / rpcf;
-    k_arp_reduce<<<(N + 255) / 256, 256, 0, st>>>(a.part, nparts, N, M, a.hmax, a.arp);
-    ISAR_COUNT(1);
+    if ((e = launch_after(a.overlap, k_arp_reduce, (N + 255) / 256, 256, 0, st, a.part, nparts, N, M, a.hmax, a.arp)))
+        return e;
     return cudaGetLastError();
 }
 
@@ -1501,15 +1502,15 @@ cudaError_t hpc_apply(float2* x, const int64_t* hq, int M, int N, cudaStream_t s
     return cudaGetLastError();
 }
 
-cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec, float2* cut, cudaStream_t st)
+cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec, float2* cut, cudaStream_t st,
+                       bool overlap)
 {
     static PerDevice attr;   // k_center's shared-memory limit, set once per device
     const int ar = attr.get([]() -> int { return -(int)center_prepare_current_device(); });
     if (ar < 0) return (cudaError_t)(-ar);
-    k_center<<<1, 1024, 3 * N * sizeof(float), st>>>(arp, y, N, 30, dec);
-    ISAR_COUNT(1);
-    k_cut<<<M, 256, 0, st>>>(y, N, dec, cut);
-    ISAR_COUNT(1);
+    cudaError_t e;
+    if ((e = launch_after(overlap, k_center, 1, 1024, 3 * N * sizeof(float), st, arp, y, N, 30, dec))) return e;
+    if ((e = launch_after(overlap, k_cut, M, 256, 0, st, y, N, dec, cut))) return e;
     return cudaGetLastError();
 }
 
