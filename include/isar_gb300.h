@@ -96,8 +96,8 @@ typedef struct {
  * Launch parameters of one context (no counterpart in the reference, whose
  * parameters are compile-time constants).  Defaults reproduce the reference:
  * 120 autofocus iterations, no stop criterion; the default autofocus engine
- * is the fastest measured for one frame of M pulses (clusters of 4, 8, 16
- * CTAs at 128, 256, 1024 pulses, the cooperative grid at 512).
+ * is the fastest measured for one frame of M pulses (clusters of 8, 16, 16
+ * CTAs at 128, 256, 1024 pulses, engine 0 at 512).
  */
 typedef struct {
     int ra_pair_min;          /* fused pair kernel while pairs >= this (128)          */

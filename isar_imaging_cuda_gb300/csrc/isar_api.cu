@@ -642,12 +642,13 @@ ISAR_API int isar_create(isar_ctx** out, const isar_radar* radar, int device, vo
         return rc;
     }
     // Default autofocus engine: the fastest for one frame of M pulses,
-    // measured on a GB300 with the reference's 120 iterations (U = 64..128
-    // selected bins): clusters of 4 / 8 CTAs at 128 / 256 pulses, the
-    // cooperative grid at 512, clusters of 16 at 1024; the cooperative grid
-    // where the device cannot launch that cluster.  Every engine computes
-    // the reference's iteration (the same parity bar).
-    const int pref = M == 128 ? 4 : M == 256 ? 8 : M == 1024 ? 16 : 0;
+    // measured on a GB300 per iteration at U = 64 selected bins: clusters of
+    // 8 CTAs at 128 pulses (1.5 us; 4 CTAs 1.9, 16 CTAs 1.6), of 16 at 256
+    // (1.6; 8 CTAs 1.9) and at 1024 (4.2; 8 CTAs 5.8), engine 0 at 512 (a
+    // cluster of 16, or the cooperative grid for the largest U); engine 0 where
+    // the device cannot launch that cluster.  Every engine computes the
+    // reference's iteration (the same parity bar).
+    const int pref = M == 128 ? 8 : M == 512 ? 0 : 16;
     c->af_cluster = (pref > 0 && isar::af_cluster_max(M) >= pref) ? pref : 0;
     *out = c;
     return ISAR_OK;
