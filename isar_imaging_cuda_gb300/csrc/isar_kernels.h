@@ -109,7 +109,7 @@ struct FEArgs {
     double* H;               // [512]
     int* bins;               // [512]
     float2* sig_part;        // [M][128] autofocus partial row sums
-    float2* gcol;            // [512][M] gathered bin columns (cluster engine, M = 1024)
+    float2* gcol;            // [512][M] gathered bin columns (cluster engine)
     unsigned* bar;           // [0] grid-barrier counter, [1] barrier timeout flag
     BarrierTest bar_test;    // poll limit and target offset of the grid barrier
     const float2* tw;
