@@ -997,8 +997,8 @@ ISAR_API int isar_pulse_compress(isar_ctx* c, const int16_t* d_ad, int iq_len, c
         }
         // the chirp's fixed factors (S per context), then the spectra
         TRY(dalloc(c, &c->d_pc_spec, base_len + need));
-        c->pc_spec_len = need;
         CU(isar::pulse_base(c->d_pc_spec, S, (float)c->r.Tp, c->st));
+        c->pc_spec_len = need;
     }
     isar::PCArgs a{};
     a.pulses = pulses;
