@@ -235,10 +235,11 @@ ISAR_API int isar_set_ra_shifts(isar_ctx* ctx, const float* shifts);
 
 /* Test hook for the bounded device waits that replace the reference's
  * exit() on a CUDA error (helper_cuda.h:583-595): the cooperative autofocus
- * engine's grid barrier gives up after `polls` polls (0 = the default limit,
- * about a second) and, with never_complete != 0, waits for one arrival more
- * than the grid makes, so that every CTA gives up, sets the timeout flag and
- * leaves the kernel.  The frame then reports ISAR_ECUDA and the context stays
+ * engine's grid barrier and the cluster engine's message waits give up after
+ * `polls` polls (0 = the default limit, about a second) and, with
+ * never_complete != 0, wait for one arrival (16 bytes) more than is sent, so
+ * that every CTA gives up, sets the timeout flag and leaves the kernel.  The
+ * frame then reports ISAR_ECUDA and the context stays
  * usable.  (0, 0) restores normal operation. */
 ISAR_API int isar_test_barrier_timeout(isar_ctx* ctx, unsigned polls, int never_complete);
 

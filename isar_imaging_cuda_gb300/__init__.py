@@ -294,8 +294,9 @@ class Context:
         _check(self._lib.isar_set_ra_shifts(self._h, self._given.ctypes.data), "isar_set_ra_shifts")
 
     def test_barrier_timeout(self, polls=0, never_complete=False):
-        """Test hook: the autofocus grid barrier polls at most `polls` times
-        and, with never_complete, waits for an arrival that never comes."""
+        """Test hook: the autofocus grid barrier and cluster messages are
+        polled at most `polls` times and, with never_complete, waited for in
+        vain."""
         _check(self._lib.isar_test_barrier_timeout(self._h, int(polls), int(bool(never_complete))),
                "isar_test_barrier_timeout")
 

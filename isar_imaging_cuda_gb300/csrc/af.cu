@@ -558,6 +558,8 @@ struct AFFrame {
     float2* gcol;          // [U][M] scratch: contiguous copy of the bin columns
     unsigned* err;         // set when a message between the CTAs does not arrive
     int max_u;             // the kernel leaves frames with more bins alone
+    unsigned polls;        // limit of a message wait
+    unsigned extra;        // bytes expected beyond those sent (test hook)
 };
 
 // The DFT over q (q = lane mod Q) of the elements c = 0..P-1 that Q
@@ -634,10 +636,11 @@ struct AfCross {
 };
 
 // One mbarrier per message direction, one arrival (the receiver's own
-// expect_tx) and the message's bytes per phase.  Waits are bounded: one that
-// runs out sets *err and `dead`, after which no wait of the CTA waits again
-// and the kernel runs to its end (the host reports the frame as failed).
+// expect_tx) and the message's bytes per phase.  Waits are bounded (leg()
+// below says how a CTA goes on after one has run out); kMsgDrainLimit polls
+// are the limit of its last wait for messages still in flight.
 constexpr unsigned kMsgWaitLimit = 1u << 20;
+constexpr unsigned kMsgDrainLimit = 1u << 12;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ uint32_t cluster_addr(uint32_t a, int rank)
@@ -666,9 +669,9 @@ __device__ __forceinline__ void msg_send2(uint32_t dst, uint32_t bar, float2 a, 
                  "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "r"(bar)
                  : "memory");
 }
-__device__ __forceinline__ void msg_wait(uint64_t* bar, uint32_t parity, volatile int* dead, unsigned* err)
+__device__ __forceinline__ bool msg_wait(uint64_t* bar, uint32_t parity, unsigned polls)
 {
-    for (unsigned i = 0; i < kMsgWaitLimit; ++i) {
+    for (unsigned i = 0; i < polls; ++i) {
         uint32_t done;
         asm volatile("{\n .reg .pred p;\n"
                      " mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
@@ -676,11 +679,9 @@ __device__ __forceinline__ void msg_wait(uint64_t* bar, uint32_t parity, volatil
                      : "=r"(done)
                      : "r"(smem_u32(bar)), "r"(parity)
                      : "memory");
-        if (done) return;
-        if (*dead) return;
+        if (done) return true;
     }
-    *dead = 1;
-    atomicOr(err, 1u);
+    return false;
 }
 
 // T -> T |T|; an exact zero stays zero.
@@ -731,7 +732,6 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     const int r = (int)cl.block_rank();
     extern __shared__ float4 dyn_smem[];
     __shared__ __align__(8) uint64_t bar_part, bar_ph;          // partial sums, phase slices arrived
-    __shared__ int dead;
     float2* ph = reinterpret_cast<float2*>(dyn_smem);          // [M]
     float2* buf = ph + M;                                       // [CL][bs] partial sums of this CTA's rows
     float2* tiles = buf + A::BUF;                               // [BINS][TILE]
@@ -743,7 +743,6 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     const int slot = tid / L, l = tid & (L - 1);                // bin within a round, lane within the bin
     const int k1 = l / Q, q = l & (Q - 1);
     if (tid == 0) {
-        dead = 0;
         msg_init(&bar_part);
         msg_init(&bar_ph);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -811,10 +810,19 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     };
     int nsweep = 0;
     uint32_t par = 0;   // phase parity of both mbarriers: bit 0 bar_part, bit 1 bar_ph
+    unsigned polls = f.polls;   // 0 once one of this thread's waits has run out
+    auto await = [&](uint64_t* bar, uint32_t bit) {
+        if (msg_wait(bar, (par & bit) ? 1u : 0u, polls)) {
+            par ^= bit;
+        } else {
+            polls = 0;
+            atomicOr(f.err, 1u);
+        }
+    };
 
     // One sweep over this CTA's bins with the phase in ph: entropy sums
     // (s1, s2, only when `ent`) and the partial row sums of the update, sent
-    // to the CTAs that own the rows.
+    // to the CTAs that own the rows (by threads whose waits have not run out).
     auto sweep = [&](bool ent, float& s1, float& s2) {
         float2 pacc[P];
 #pragma unroll
@@ -913,6 +921,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
             for (int i = 0; i < P; ++i) ta[l + L * i] = make_float2(pacc[i].x * invM, pacc[i].y * sy);
         }
         __syncthreads();
+        if (polls == 0) return;
         for (int m = 2 * tid; m < M; m += 2 * A::THREADS) {
             float2 a = make_float2(0.0f, 0.0f), b = a;
 #pragma unroll
@@ -929,10 +938,13 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     };
 
     // Entropy of the selected bins, in two halves around a cluster barrier:
-    // this CTA's sums (s1 = sum p, s2 = sum p log2 p) into red[32..33], then
-    // after the barrier warp 0 adds the CL CTAs' sums (one remote read per
-    // lane, a fixed-order tree: every CTA gets the same value) and returns
-    // ln S1 - ln 2 * S2 / S1 in lane 0 of warp 0.
+    // this CTA's sums (s1 = sum p, s2 = sum p log2 p) into one of two slots,
+    // red[32..33] and red[34..35] in turn, then after the barrier warp 0 adds
+    // the CL CTAs' sums (one remote read per lane, a fixed-order tree: every CTA
+    // gets the same value) and returns ln S1 - ln 2 * S2 / S1 in lane 0 of warp 0.
+    // A CTA writes a slot again after the next barrier, which no CTA passes
+    // before all have read it.
+    int eslot = 32;
     auto entropy_part = [&](float s1, float s2) {
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
@@ -950,16 +962,16 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
                 a1 += red[w];
                 a2 += red[16 + w];
             }
-            red[32] = a1;
-            red[33] = a2;
+            red[eslot] = a1;
+            red[eslot + 1] = a2;
         }
     };
     auto entropy_total = [&]() {   // warp 0, after the cluster barrier
         double S1 = 0.0, S2 = 0.0;
         if (lane < CL) {
             const double* rr = cl.map_shared_rank(red, lane);
-            S1 = rr[32];
-            S2 = rr[33];
+            S1 = rr[eslot];
+            S2 = rr[eslot + 1];
         }
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) {
@@ -972,6 +984,14 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     // One autofocus run from the phase in ph: up to `iters` updates, fewer
     // when the stop criterion ends it.  Returns, in warp 0, the entropy at the
     // last evaluated phase.
+    //
+    // A thread whose wait has run out waits no more, sends no message and, thread
+    // 0, expects none: a phase that has not completed gets no second arrival,
+    // and at most one phase's bytes come unexpected.  The peers then miss its
+    // messages and run out in the same way; whoever does not can only be one whose
+    // messages are all there.  All threads go on through the sweeps and their
+    // barriers and meet at every cluster barrier, whose number depends only on
+    // the iteration count and on the entropies, the same in all CTAs.
     auto leg = [&](float ltol, int& used) -> float {
         float e_prev = 0.0f, e_last = 0.0f;   // meaningful in warp 0
         used = iters;
@@ -985,7 +1005,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
             bool stop = false;
             if (need_e) {
                 entropy_part(s1, s2);
-                cl.sync();   // red[32..33] of every CTA are complete
+                cl.sync();   // the slots of every CTA are complete
                 if (warp == 0) {
                     const float E = entropy_total();
                     if (check) {
@@ -997,10 +1017,10 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
                 }
                 __syncthreads();
                 stop = red[40] != 0.0;
+                eslot ^= 2;
             }
-            if (tid == 0) msg_expect(&bar_part, M * sizeof(float2));
-            msg_wait(&bar_part, par & 1, &dead, f.err);
-            par ^= 1;
+            if (tid == 0 && polls > 0) msg_expect(&bar_part, M * sizeof(float2) + f.extra);
+            await(&bar_part, 1u);
             if (stop) {
                 cl.sync();   // every CTA has these messages: the next leg may send
                 used = it;
@@ -1021,16 +1041,27 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
                     s = cadd(s, t);
                 }
                 s = unit(s);
+                if (polls > 0) {
 #pragma unroll
-                for (int x = 0; x < CL; x += tpr)
-                    msg_send(cluster_addr(smem_u32(&ph[r * rows + ml]), part + x),
-                             cluster_addr(smem_u32(&bar_ph), part + x), s);
+                    for (int x = 0; x < CL; x += tpr)
+                        msg_send(cluster_addr(smem_u32(&ph[r * rows + ml]), part + x),
+                                 cluster_addr(smem_u32(&bar_ph), part + x), s);
+                }
             }
-            if (tid == 0) msg_expect(&bar_ph, M * sizeof(float2));
-            msg_wait(&bar_ph, par >> 1, &dead, f.err);
-            par ^= 2;
+            if (tid == 0 && polls > 0) msg_expect(&bar_ph, M * sizeof(float2));
+            await(&bar_ph, 2u);
         }
         return e_last;
+    };
+    // No CTA leaves while another may still send to it.  One that has received
+    // all it waited for is done once the others send no more (the barrier); one
+    // that gave up waits again, with a limit, for messages still in flight.
+    auto leave = [&]() {
+        cl.sync();
+        if (polls == 0) {
+            msg_wait(&bar_part, par & 1u, kMsgDrainLimit);
+            msg_wait(&bar_ph, par >> 1, kMsgDrainLimit);
+        }
     };
 
     if (!f.alt) {
@@ -1041,7 +1072,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
             f.stat[0] = used;
             f.stat[1] = __float_as_int(e);
         }
-        cl.sync();   // no CTA leaves while another may still send to it
+        leave();
         return;
     }
     // the learned leg, then the plain leg (one copy of the code)
@@ -1073,7 +1104,7 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
         f.stat[5] = used[1];
         f.stat[6] = used[0];
     }
-    cl.sync();   // no CTA leaves while another may still send to it
+    leave();
 }
 
 // cut[m][c] *= phase[m]  (phase_adjustment.cu:324)
@@ -1172,7 +1203,8 @@ static cudaError_t af_cluster_launch(const FEArgs& a, int cl, int max_u, cudaStr
     if (cl > mx) return cudaErrorInvalidClusterSize;
     cudaLaunchAttribute at[2];
     const cudaLaunchConfig_t cfg = af_cluster_config<M>(cl, a.overlap != 0, st, at);
-    AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol, a.bar + 3, max_u};
+    AFFrame fr{a.cut, a.bins, a.fdec, a.phase, a.af_stat, a.ws_w ? a.ws_phase : nullptr, a.gcol, a.bar + 3, max_u,
+               a.bar_test.limit == kSpinLimit ? kMsgWaitLimit : (unsigned)a.bar_test.limit, a.bar_test.extra ? 16u : 0u};
     cudaError_t e = cudaLaunchKernelEx(&cfg, af_kernel<M>(cl), fr, a.iters, a.tol, a.tw);
     if (e == cudaSuccess) ISAR_COUNT(1);
     return e;

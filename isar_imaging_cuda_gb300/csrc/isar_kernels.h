@@ -90,6 +90,8 @@ struct RAArgs {
 // Poll limit of the autofocus grid barrier (about a second of polling), and
 // the test hook that makes it run out: `extra` arrivals are added to every
 // barrier's target, so no CTA can pass and each gives up after `limit` polls.
+// The cluster engine's message waits take a changed limit too, and expect 16
+// bytes that are not sent while `extra` is set.
 constexpr unsigned long long kSpinLimit = 1ull << 22;
 struct BarrierTest {
     unsigned long long limit = kSpinLimit;
