@@ -96,17 +96,18 @@ typedef struct {
  * Launch parameters of one context (no counterpart in the reference, whose
  * parameters are compile-time constants).  Defaults reproduce the reference:
  * 120 autofocus iterations, no stop criterion; the default autofocus engine
- * is the fastest measured for one frame of M pulses (clusters of 8, 16, 16
- * CTAs at 128, 256, 1024 pulses, engine 0 at 512).
+ * is the fastest measured for one frame of M pulses and 64 selected bins
+ * (clusters of 8, 16, 16 CTAs at 128, 256, 1024 pulses).  At 512 pulses a
+ * context reports af_cluster 0 and picks, frame by frame, a cluster of 16 or
+ * (more than 256 bins) the grid until isar_set_tuning names an engine; both
+ * agree within the parity bar, not bit for bit.
  */
 typedef struct {
     int ra_pair_min;          /* fused pair kernel while pairs >= this (128)          */
     int ra_rows_per_cta;      /* rows per CTA of the envelope accumulation (4)        */
     int ra_rows_final;        /* rows per CTA of the final range transform (4)        */
     int af_cluster;           /* autofocus engine: 0 = one cooperative grid of 128    */
-                              /* CTAs (up to 512 pulses a cluster of 16 where one can */
-                              /* be launched: same results, no stop criterion);       */
-                              /* 4, 8, 16 = one thread-block cluster per frame        */
+                              /* CTAs; 4, 8, 16 = one thread-block cluster per frame  */
     float af_tol;             /* stop once the entropy of the selected bins changes   */
                               /* by <= af_tol * |entropy| per iteration (mean over 4, */
                               /* checked every 4th iteration; cluster engine; 0 = off)*/

@@ -1272,19 +1272,13 @@ static cudaError_t fe_run_m(const FEArgs& a, cudaStream_t st)
         if ((e = nn::forward(*a.ws_w, *a.ws_a, 1, M, a.ws_err, st))) return e;
         if ((e = nn::ws_phase(a.ws_psi, a.ws_a->out, M, a.ws_phase, st))) return e;
     }
-    // Engine 0 up to 512 pulses runs as one 16-CTA cluster where one can be
-    // launched: per iteration, cooperative grid -> cluster, U = 64 and 256:
-    // 6.4 -> 1.6 and 6.5 -> 2.1 us at 128 pulses, 6.5 -> 1.6 and 6.5 -> 3.1 at 256,
-    // 7.6 -> 2.8 and 7.8 -> 6.0 at 512.  Only at 512 pulses and the largest U,
+    // The choice by bins (512 pulses): a cluster of 16 takes 2.8 us per iteration
+    // at U = 64 and 6.0 at U = 256, the grid 7.6 and 7.8; only at the largest U,
     // 512 (profiles below one count: the integer mean of the threshold is 0), is
-    // the grid ahead (8 against 10 us): both kernels are launched there and the
-    // one that the frame's U does not select returns at once.  At 1024 pulses
-    // the grid is ahead from U = 256 (9.0 against 9.9; 8.2 against 4.2 at U = 64)
-    // and engine 0 stays the grid, as it does under the barrier's test hook.
-    const bool auto16 =
-        a.af_cluster == 0 && M <= 512 && !a.bar_test.active() && af_cluster_setup<M>() >= 16;
-    const int cl = auto16 ? 16 : a.af_cluster;
-    const int max_u = auto16 && M == 512 ? 256 : C;
+    // the grid ahead (8 against 10).  U is known on the device only: both kernels
+    // are launched and the one that it does not select returns at once.
+    const int cl = a.af_auto ? 16 : a.af_cluster;
+    const int max_u = a.af_auto ? 256 : C;
     if (a.iters > 0 && cl > 0) {
         if ((e = af_cluster_launch<M>(a, cl, max_u, st))) return e;
     }

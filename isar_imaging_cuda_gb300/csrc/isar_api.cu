@@ -197,6 +197,7 @@ struct isar_ctx {
     bool use_graphs = true;
     bool overlap = true;           // kernels overlap their predecessors' ends (launch.cuh)
     bool reset_node = false;       // RAArgs::reset_node
+    bool af_auto = false;          // FEArgs::af_auto; af_cluster is 0
     std::vector<CachedGraph> graphs;
     unsigned long long graph_tick = 0;
     // learned warm start: the attached network and this context's
@@ -217,6 +218,8 @@ void isar::set_lane(isar_ctx* c, bool reset_node)
     c->overlap = false;
     c->reset_node = reset_node;
 }
+bool isar::engine_auto(const isar_ctx* c) { return c->af_auto; }
+void isar::set_engine_auto(isar_ctx* c) { c->af_auto = true; }
 
 namespace {
 
@@ -413,6 +416,7 @@ isar::FEArgs fe_args(isar_ctx* c, float2* cut, int iters)
     a.bar_test = c->bar_test;
     a.tw = c->d_tw;
     a.af_cluster = c->af_cluster;
+    a.af_auto = c->af_auto;
     a.tol = c->af_tol;
     a.af_stat = c->d_fdec + 4;
     a.overlap = c->overlap;
@@ -644,12 +648,15 @@ ISAR_API int isar_create(isar_ctx** out, const isar_radar* radar, int device, vo
     // Default autofocus engine: the fastest for one frame of M pulses,
     // measured on a GB300 per iteration at U = 64 selected bins: clusters of
     // 8 CTAs at 128 pulses (1.5 us; 4 CTAs 1.9, 16 CTAs 1.6), of 16 at 256
-    // (1.6; 8 CTAs 1.9) and at 1024 (4.2; 8 CTAs 5.8), engine 0 at 512 (a
-    // cluster of 16, or the cooperative grid for the largest U); engine 0 where
-    // the device cannot launch that cluster.  Every engine computes the
-    // reference's iteration (the same parity bar).
-    const int pref = M == 128 ? 8 : M == 512 ? 0 : 16;
-    c->af_cluster = (pref > 0 && isar::af_cluster_max(M) >= pref) ? pref : 0;
+    // (1.6; 8 CTAs 1.9) and at 1024 (4.2; 8 CTAs 5.8); at 512 the choice by bins
+    // (fe_run_m), reported as engine 0; the cooperative grid where the device
+    // cannot launch that cluster.  (At 1024 pulses the grid is ahead from 256
+    // bins, 9.0 against 9.9 us.)  Every engine computes the reference's iteration
+    // (the same parity bar).
+    const int pref = M == 128 ? 8 : 16;
+    const bool can = isar::af_cluster_max(M) >= pref;
+    c->af_auto = can && M == 512;
+    c->af_cluster = can && M != 512 ? pref : 0;
     *out = c;
     return ISAR_OK;
 }
@@ -897,6 +904,7 @@ ISAR_API int isar_set_tuning(isar_ctx* c, const isar_tuning* t)
     c->ra_rpc = t->ra_rows_per_cta;
     c->ra_rpc_final = t->ra_rows_final;
     c->af_cluster = t->af_cluster;
+    c->af_auto = false;
     c->af_tol = t->af_tol;
     c->af_iters = t->af_iters;
     for (auto& g : c->graphs) cudaGraphExecDestroy(g.exec);

@@ -286,6 +286,7 @@ ISAR_API int isar_autotune(isar_ctx* c, const float* d_echo, const double* d_vel
     if ((engines & 3) == 0) return fail(ISAR_EINVAL, "engines must allow the cooperative (1) or cluster (2) engine");
     isar_tuning base;
     TRY(isar_get_tuning(c, &base));
+    const bool was_auto = isar::engine_auto(c);
     cudaStream_t st = static_cast<cudaStream_t>(isar_stream(c));
     // scratch image of the largest frame (echo_num <= 1024); tuning is a
     // set-up step, not the imaging path
@@ -359,6 +360,7 @@ ISAR_API int isar_autotune(isar_ctx* c, const float* d_echo, const double* d_vel
     cudaFree(d_img);
     if (rc != ISAR_OK) {
         isar_set_tuning(c, &base);
+        if (was_auto) isar::set_engine_auto(c);
         return rc;
     }
     TRY(isar_set_tuning(c, &best));

@@ -96,7 +96,6 @@ constexpr unsigned long long kSpinLimit = 1ull << 22;
 struct BarrierTest {
     unsigned long long limit = kSpinLimit;
     unsigned extra = 0;
-    bool active() const { return limit != kSpinLimit || extra != 0; }
 };
 
 struct FEArgs {
@@ -115,11 +114,11 @@ struct FEArgs {
     unsigned* bar;           // [0] grid-barrier counter, [1] barrier timeout flag
     BarrierTest bar_test;    // poll limit and target offset of the grid barrier
     const float2* tw;
-    // Autofocus engine: 4, 8 or 16 = one thread-block cluster of that many
-    // CTAs per frame (distributed shared memory, no grid barrier); 0 = one
-    // cooperative grid (128 CTAs, grid barriers) or, up to 512 pulses, a
-    // cluster of 16 where one can be launched, without a stop criterion.
+    // Autofocus engine: 0 = one cooperative grid (128 CTAs, grid barriers);
+    // 4, 8 or 16 = one thread-block cluster of that many CTAs per frame
+    // (distributed shared memory, no grid barrier).
     int af_cluster;
+    int af_auto;             // a cluster of 16 or the grid by the frame's bin count instead
     // Entropy stop criterion (cluster engine): stop once the entropy of the
     // selected bins changes by <= tol * |entropy| per iteration (mean over
     // the 4 iterations between two checks); 0 runs all `iters` (the
@@ -218,6 +217,10 @@ cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec
 // Makes the context a batch's lane: its kernels do not overlap their
 // predecessors' ends (launch.cuh), and RAArgs::reset_node is set as given.
 void set_lane(isar_ctx* c, bool reset_node);
+// Whether the context still chooses its autofocus engine per frame (the default
+// at 512 pulses, until isar_set_tuning), and that choice restored.
+bool engine_auto(const isar_ctx* c);
+void set_engine_auto(isar_ctx* c);
 // Raises k_center's dynamic shared-memory limit to the kMaxN case on the
 // calling thread's current device (the attribute is per device).
 cudaError_t center_prepare_current_device();

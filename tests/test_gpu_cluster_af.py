@@ -91,10 +91,9 @@ def test_cluster_few_and_many_bins(torch_cuda, gb300, M, cl, bright, U, iters):
     assert rel_l2(got, want) < TOL_IMG
 
 
-# Engine 0 picks its kernel by the pulse count and, at 512 pulses, by U on the
-# device: 256 bins on the cluster, 512 (profiles below one count, whose
-# integer mean is 0) on the cooperative grid.  Both give the oracle's result
-# and leave the trace's engine fields as engine 0 reports them.
+# Engine 0, the cooperative grid, from few bins to 512 (profiles below one
+# count, whose integer mean is 0): the oracle's result, and the trace's engine
+# fields as engine 0 reports them.
 @pytest.mark.parametrize("M", [128, 256, 512, 1024])
 @pytest.mark.parametrize("bright,scale,U", [(40, 6000.0, 32), (280, 6000.0, 256), (512, 0.5, 512)])
 def test_engine0_every_bin_count(torch_cuda, gb300, M, bright, scale, U):
@@ -113,6 +112,40 @@ def test_engine0_every_bin_count(torch_cuda, gb300, M, bright, scale, U):
         tr = ctx.trace()
     assert tr["unit2_num"] == U and np.isnan(tr["af_entropy"])
     assert rel_l2(got, want) < TOL_IMG
+
+
+# af_cluster 0 names the cooperative grid at every size (a poll limit of its own
+# does not change the engine), and a 512-pulse context that was never tuned
+# picks by bins: the 16-CTA cluster up to 256, the grid above.
+@pytest.mark.parametrize("M", [128, 256, 512])
+@pytest.mark.parametrize("bright,scale,U", [(40, 6000.0, 32), (280, 6000.0, 256), (512, 0.5, 512)])
+def test_engine0_is_the_grid_and_the_default_picks_by_bins(torch_cuda, gb300, M, bright, scale, U):
+    torch = torch_cuda
+    rng = np.random.default_rng(5 * M + bright)
+    cut = (rng.standard_normal((M, 512)) + 1j * rng.standard_normal((M, 512))).astype(np.complex64) * scale / 60
+    k = (512 - bright) // 2
+    cut[:, k:k + bright] = (scale * np.exp(2j * np.pi * rng.random((M, bright)))).astype(np.complex64)
+
+    def run(cl=None, polls=0):
+        with ctx_for(gb300, torch, M, 2048) as ctx:
+            if cl is not None:
+                _cluster_or_skip(ctx, cl)
+                ctx.set_tuning(af_cluster=cl)
+            ctx.test_barrier_timeout(polls, False)
+            dc = to_dev(torch, cut)
+            ctx.stage_fast_entropy(dc, 6)
+            out = from_dev(torch, dc)
+            tr = ctx.trace()
+        assert tr["unit2_num"] == U
+        return out, np.isnan(tr["af_entropy"])
+
+    grid, none = run(0)
+    assert none and np.array_equal(grid, run(0, polls=1 << 21)[0])
+    cluster, none = run(16)
+    assert not none and not np.array_equal(cluster, grid)
+    if M == 512:
+        out, none = run()
+        assert none and np.array_equal(out, cluster if U <= 256 else grid)
 
 
 def test_cluster_stop_criterion_equals_oracle_at_same_count(torch_cuda, gb300):

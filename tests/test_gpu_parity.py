@@ -118,8 +118,8 @@ def test_center_cut_stage(torch_cuda, gb300, M, N):
     assert rel_l2(cut, cut_want) < 1e-5
 
 
-# af_cluster 0: the cooperative engine (k_af_persist, the single-frame
-# default); 16: the cluster engine (k_af_cluster_w1024 at 1024 pulses).
+# af_cluster 0: the cooperative engine (k_af_persist); 16: the cluster engine
+# (k_af_cluster).
 @pytest.mark.parametrize("M,N,seed,af_cluster", [(128, 512, 1, 0), (256, 1024, 2, 0), (512, 2048, 3, 0),
                                                  (1024, 8192, 4, 0), (1024, 8192, 4, 16), (1024, 2048, 5, 0)])
 def test_fast_entropy_stage(torch_cuda, gb300, M, N, seed, af_cluster):
@@ -166,7 +166,7 @@ def test_post_stage(torch_cuda, gb300, M, mtrc, ifds):
 
 # (256, 4096, plain) is the plain single-frame workload; (1024, 8192, full)
 # the five-stage benchmark workload (HPC + MTRC), with the cooperative
-# autofocus engine (af_cluster 0, the plain pipeline's) and the cluster engine.
+# autofocus engine (af_cluster 0) and the cluster engine.
 @pytest.mark.parametrize("M,N,full,seed,af_cluster", [(128, 512, False, 31, 0), (256, 4096, False, 32, 0),
                                                       (256, 2048, True, 33, 0), (256, 4096, False, 42, 0),
                                                       (1024, 8192, True, 41, 0), (1024, 8192, True, 41, 16),
