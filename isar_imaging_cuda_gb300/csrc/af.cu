@@ -703,7 +703,7 @@ __device__ __forceinline__ float2 unit(float2 s)
 {
     const float p = s.x * s.x + s.y * s.y;
     float y = rsqrtf(p);
-    if (p > 0.0f && p < CUDART_INF_F) y = fmaf(y, fmaf(-0.5f * p * y, y, 0.5f), y);
+    if (p > 0.0f && p < CUDART_INF_F) y = fmaf(y, fmaf(-0.5f * y * p, y, 0.5f), y);   // y first: p / 2 may round
     return make_float2(s.x * y, s.y * y);
 }
 

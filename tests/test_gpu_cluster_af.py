@@ -148,6 +148,30 @@ def test_engine0_is_the_grid_and_the_default_picks_by_bins(torch_cuda, gb300, M,
         assert none and np.array_equal(out, cluster if U <= 256 else grid)
 
 
+# Row sums whose |s|^2 is a handful of the smallest float: it carries two
+# roundings of half a unit, so at one unit s / |s| may be as long as sqrt(2), but
+# the normalisation adds no error of its own.
+@pytest.mark.parametrize("M", [128, 512, 1024])
+def test_cluster_normalises_the_smallest_sums(torch_cuda, gb300, M):
+    torch = torch_cuda
+    rng = np.random.default_rng(M)
+    base = np.exp(2j * np.pi * rng.random((M, 512)))
+    a0 = (4e-23 / (512 * 1.3 * np.sqrt(M))) ** (1.0 / 3.0)   # |s| ~ 512 bins a^3 sqrt(M)
+    seen = 0
+    with ctx_for(gb300, torch, M, 2048) as ctx:
+        _cluster_or_skip(ctx, 8)
+        ctx.set_tuning(af_cluster=8)
+        for k in range(-4, 5):
+            dc = to_dev(torch, (base * a0 * 1.12 ** k).astype(np.complex64))
+            ctx.stage_fast_entropy(dc, 1)
+            torch.cuda.synchronize()
+            r = np.abs(ctx.trace()["phase"].astype(np.complex128))
+            r = r[np.isfinite(r)]
+            seen += np.count_nonzero(np.abs(r - 1.0) > 0.1)   # sums of a few units are there
+            assert np.all(r < np.sqrt(2.0) * (1.0 + 1e-5))
+    assert seen > M // 16
+
+
 def test_cluster_stop_criterion_equals_oracle_at_same_count(torch_cuda, gb300):
     torch = torch_cuda
     M, N = 256, 1024
