@@ -64,8 +64,9 @@ __device__ __forceinline__ float2 twc_mul(float2 d, int j, int R)
 // differences are packed pairs.  SRC: the inputs come from a caller's functor
 // and may be products; the first stage then stays scalar, where the compiler
 // fuses such a product into the sum (one rounding less), as the envelopes of
-// the range alignment have always been rounded.
-template <int R, bool INV, bool SRC = false>
+// the range alignment have always been rounded.  PACK = false: all scalar, for
+// kernels that spill on the register pairs.
+template <int R, bool INV, bool SRC = false, bool PACK = true>
 __device__ __forceinline__ void dft_reg(float2* a)
 {
 #pragma unroll
@@ -76,7 +77,7 @@ __device__ __forceinline__ void dft_reg(float2* a)
 #pragma unroll
             for (int k = 0; k < half; ++k) {
                 float2 u = a[s + k], v = a[s + k + half];
-                if (SRC && len == R) {
+                if (!PACK || (SRC && len == R)) {
                     a[s + k] = make_float2(u.x + v.x, u.y + v.y);
                     a[s + k + half] = twc_mul<INV>(make_float2(u.x - v.x, u.y - v.y), k * (R / len), R);
                 } else {
@@ -209,7 +210,7 @@ __device__ __forceinline__ void fft_twiddle16(float2* v, int k, const Tw& tw)
     }
 }
 
-template <int N, int R, int NS, bool INV, bool FIRST, bool LAST, class Src, class Dst, class Tw, class Hook>
+template <int N, int R, int NS, bool INV, bool FIRST, bool LAST, bool PACK, class Src, class Dst, class Tw, class Hook>
 __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt, const Tw& tw, bool active,
                                          Hook& hook)
 {
@@ -250,7 +251,7 @@ __device__ __forceinline__ void fft_pass(Src& src, Dst& dst, float2* sm, int lt,
                     v[b * R + r] = cmul(v[b * R + r], w);
                 }
             }
-            dft_reg<R, INV, FIRST>(&v[b * R]);
+            dft_reg<R, INV, FIRST, PACK>(&v[b * R]);
             const int base = (j / NS) * NS * R + k;
             const int pb = fpad(base);
 #pragma unroll
@@ -313,18 +314,20 @@ __device__ __forceinline__ void fft_last16x2(Dst& dst, float2* sm, int lt, const
     __syncthreads();
 }
 
-template <int N, bool INV, int PASS, int NS, class Src, class Dst, class Tw, class Hook>
+template <int N, bool INV, bool PACK, int PASS, int NS, class Src, class Dst, class Tw, class Hook>
 __device__ __forceinline__ void fft_passes(Src& src, Dst& dst, float2* sm, int lt, const Tw& tw, bool active,
                                            Hook& hook)
 {
     using S = FFTShape<N>;
     constexpr int R = (PASS < S::NP16) ? 16 : (1 << S::REM);
     if constexpr (S::FUSE2 && PASS == S::NP16 - 1) {
+        static_assert(PACK, "the joined pass is packed");
         fft_last16x2<N, INV>(dst, sm, lt, tw, active);
         return;
     }
-    fft_pass<N, R, NS, INV, PASS == 0, PASS == S::NPASS - 1>(src, dst, sm, lt, tw, active, hook);
-    if constexpr (PASS + 1 < S::NPASS) fft_passes<N, INV, PASS + 1, NS * R>(src, dst, sm, lt, tw, active, hook);
+    fft_pass<N, R, NS, INV, PASS == 0, PASS == S::NPASS - 1, PACK>(src, dst, sm, lt, tw, active, hook);
+    if constexpr (PASS + 1 < S::NPASS)
+        fft_passes<N, INV, PACK, PASS + 1, NS * R>(src, dst, sm, lt, tw, active, hook);
 }
 
 // One team transform.  src(i) -> float2 for i in [0,N) (first pass, may read
@@ -336,12 +339,12 @@ __device__ __forceinline__ void fft_passes(Src& src, Dst& dst, float2* sm, int l
 // tw: the global kTwN table (TwGlobal) or a TwShared<N> accessor.
 // hook() runs in every thread once all src() reads of the CTA are done
 // (after the first pass's load barrier), e.g. to refill the source buffer.
-template <int N, bool INV, class Src, class Dst, class Tw, class Hook = NoHook>
+template <int N, bool INV, bool PACK = true, class Src, class Dst, class Tw, class Hook = NoHook>
 __device__ __forceinline__ void team_fft(Src src, Dst dst, float2* sm, int lt, const Tw& tw, bool active = true,
                                          Hook hook = Hook{})
 {
     static_assert(N >= 32 && (N & (N - 1)) == 0 && N <= kTwN, "FFT size");
-    fft_passes<N, INV, 0, 1>(src, dst, sm, lt, tw, active, hook);
+    fft_passes<N, INV, PACK, 0, 1>(src, dst, sm, lt, tw, active, hook);
 }
 
 template <int N, bool INV, class Src, class Dst>

@@ -52,14 +52,20 @@ __global__ void k_pc_base(float2* __restrict__ base, int S, float tpf)
 // 64 registers let two CTAs (four at 4096 points) share an SM, so that one's
 // loads, barriers and sine latencies hide behind the other's transforms, and
 // the Hamming window and time axis come from a table of the context (a cosine
-// and three divisions per sample and pulse before).  1024 pulses of 5000 samples:
-// 125 -> 96 us (with the global per-pass twiddles in place of the shared
-// two-level table 110: they spill at 64 registers).
+// and three divisions per sample and pulse before).  Spills at 64 registers
+// decide the rest.  Packed sums only at 8192 points (64 bytes of spills; scalar
+// 60 and slower, 100.5 against 95.6 us for 1024 pulses), scalar at 4096 (20 bytes
+// instead of 156; 1024 pulses 43.8 -> 43.1 us, 37 pulses 14.4 -> 12.4) and at
+// 16384 (4 instead of 124; 249.8 -> 227.2 us); the global per-pass twiddles in
+// place of the shared two-level table spill 400 (8192 points 110 us).  With one
+// CTA per SM and the window and axis computed per pulse 1024 pulses took 58.8,
+// 131.2 and 245.4 us.
 template <int NF>
 __global__ void __launch_bounds__(NF / 16, 1024 / (NF / 16))
 k_pulse_compress(PCArgs a)
 {
     using F = FFTShape<NF>;
+    constexpr bool PACK = NF == 8192;
     extern __shared__ float4 dyn_smem[];
     float2* sm = reinterpret_cast<float2*>(dyn_smem);
     float2* twt = sm + F::SMEM;
@@ -75,7 +81,7 @@ k_pulse_compress(PCArgs a)
     const int L = a.iq_len;
 
     // X = FFT(x): the int16 I/Q samples, zero-padded to NF
-    team_fft<NF, false>(
+    team_fft<NF, false, PACK>(
         [&](int i) {
             if (i >= L) return make_float2(0.0f, 0.0f);
             const short2 q = reinterpret_cast<const short2*>(ad)[i];
@@ -88,7 +94,7 @@ k_pulse_compress(PCArgs a)
     const float v2 = __fdiv_rn(__fmul_rn(2.0f, (float)a.vel[p]), 300000000.0f);   // LIGHT_SPEED
     const float v2c = __fsub_rn(1.0f, v2);
     const float c1 = __fdiv_rn(__fmul_rn(__fmul_rn(__fmul_rn(-2.0f, kPiF), a.fc_f), v2), v2c);
-    team_fft<NF, false>(
+    team_fft<NF, false, PACK>(
         [&](int i) { return i < a.S ? pc_ref(__ldg(&a.base[i]), v2c, c1, a.c2) : make_float2(0.0f, 0.0f); },
         [&](int k, float2 r, int) { sm[fpad(k)] = cmulc(r, sp[k]); }, sm, lt, tws);
 
@@ -96,17 +102,17 @@ k_pulse_compress(PCArgs a)
     const float inv = 1.0f / (float)NF;
     float bv = -1.0f;
     int bi = 0x7fffffff;
-    team_fft<NF, true>([&](int i) { return sm[fpad(i)]; },
-                       [&](int i, float2 v, int) {
-                           const float2 y = make_float2(v.x * inv, v.y * inv);
-                           sm[fpad(i)] = y;
-                           const float m = fabsf(y.x) + fabsf(y.y);
-                           if (m > bv || (m == bv && i < bi)) {
-                               bv = m;
-                               bi = i;
-                           }
-                       },
-                       sm, lt, tws);
+    team_fft<NF, true, PACK>([&](int i) { return sm[fpad(i)]; },
+                             [&](int i, float2 v, int) {
+                                 const float2 y = make_float2(v.x * inv, v.y * inv);
+                                 sm[fpad(i)] = y;
+                                 const float m = fabsf(y.x) + fabsf(y.y);
+                                 if (m > bv || (m == bv && i < bi)) {
+                                     bv = m;
+                                     bi = i;
+                                 }
+                             },
+                             sm, lt, tws);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
