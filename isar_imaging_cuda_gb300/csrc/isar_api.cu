@@ -196,7 +196,6 @@ struct isar_ctx {
     // cached CUDA graphs of whole frames
     bool use_graphs = true;
     bool overlap = true;           // kernels overlap their predecessors' ends (launch.cuh)
-    bool reset_node = false;       // RAArgs::reset_node
     bool af_auto = false;          // FEArgs::af_auto; af_cluster is 0
     std::vector<CachedGraph> graphs;
     unsigned long long graph_tick = 0;
@@ -213,11 +212,7 @@ struct isar_ctx {
     bool ws_alloc = false;
 };
 
-void isar::set_lane(isar_ctx* c, bool reset_node)
-{
-    c->overlap = false;
-    c->reset_node = reset_node;
-}
+void isar::set_lane(isar_ctx* c) { c->overlap = false; }
 bool isar::engine_auto(const isar_ctx* c) { return c->af_auto; }
 void isar::set_engine_auto(isar_ctx* c) { c->af_auto = true; }
 
@@ -393,7 +388,6 @@ isar::RAArgs ra_args(isar_ctx* c, const float2* x, float2* y, bool hpc, bool hrr
     a.given_shifts = c->ra_given ? 1 : 0;
     a.err = c->d_bar + 2;
     a.overlap = c->overlap;
-    a.reset_node = c->reset_node;
     return a;
 }
 

@@ -143,6 +143,7 @@ int ensure_lanes(isar_batch* b, Shape* s, int n)
         Lane l;
         int rc = isar_create(&l.ctx, &s->r, b->dev, nullptr);
         if (rc != ISAR_OK) return rc;
+        isar::set_lane(l.ctx);
         l.st = static_cast<cudaStream_t>(isar_stream(l.ctx));
         if (cudaEventCreateWithFlags(&l.done, cudaEventDisableTiming) != cudaSuccess) {
             destroy_lane(l);
@@ -205,21 +206,12 @@ int record_batch(isar_batch* b, const isar_batch_frame* f, int n, int lanes)
         for (auto& q : p.second) used += q.empty() ? 0 : 1;
         TRY(ensure_lanes(b, p.first, used));
     }
-    // Frames of one shape run through kernels alone: their lanes advance in step
-    // and the graph needs no other nodes.  Measured against one memset node per
-    // frame (32 learned frames of 1024 x 8192 14.65 -> 13.55 ms, 64 plain of
-    // 128 x 2048 2.07 -> 1.89, never slower).  Frames of several shapes are as
-    // fast or up to 10 % faster with that node, which lets lanes of unlike length
-    // drift apart (64 uneven frames 6.05 against 6.30 ms, 32 on four lanes per
-    // shape 5.5 against 6.0).
-    const bool reset_node = plan.size() > 1;
     CU(cudaEventRecord(b->fork, b->st));
     for (auto& p : plan) {
         int li = 0;
         for (auto& q : p.second) {
             if (q.empty()) continue;
             Lane& l = p.first->lanes[li++];
-            isar::set_lane(l.ctx, reset_node);
             CU(cudaStreamWaitEvent(l.st, b->fork, 0));
             for (int i : q) TRY(isar_image_device(l.ctx, f[i].d_echo, f[i].d_velocity, f[i].flags, f[i].d_img));
             CU(cudaEventRecord(l.done, l.st));

@@ -84,7 +84,6 @@ struct RAArgs {
     unsigned* err;           // set when a row-copy wait runs out (rows invalid)
     int x_iq16;              // x holds int16 I/Q pairs (level 0 reads them directly)
     int overlap;             // kernels overlap their predecessors' ends (launch.cuh)
-    int reset_node;          // the profile maximum is reset by a memset of its own (isar_batch.cpp)
 };
 
 // Poll limit of the autofocus grid barrier (about a second of polling), and
@@ -214,9 +213,9 @@ cudaError_t ra_run(const RAArgs& a, cudaStream_t st);
 cudaError_t arp_from_y(const float2* y, int M, int N, float* tmp, unsigned* hmax, float* arp, cudaStream_t st);
 cudaError_t center_cut(const float* arp, const float2* y, int M, int N, int* dec, float2* cut, cudaStream_t st,
                        bool overlap = false);
-// Makes the context a batch's lane: its kernels do not overlap their
-// predecessors' ends (launch.cuh), and RAArgs::reset_node is set as given.
-void set_lane(isar_ctx* c, bool reset_node);
+// Makes a new context a batch's lane: its kernels do not overlap their
+// predecessors' ends (launch.cuh).
+void set_lane(isar_ctx* c);
 // Whether the context still chooses its autofocus engine per frame (the default
 // at 512 pulses, until isar_set_tuning), and that choice restored.
 bool engine_auto(const isar_ctx* c);

@@ -1449,7 +1449,6 @@ static cudaError_t ra_run_n(const RAArgs& a, cudaStream_t st)
         shift_off += pairs;
         if ((e = cudaGetLastError())) return e;
     }
-    if (a.reset_node && (e = cudaMemsetAsync(a.hmax, 0, sizeof(unsigned), st))) return e;
     // final IFFT + ARP partials + hmax
     const int arp_rows = M < 256 ? M : 256;
     int rpcf = a.rpc_final;
