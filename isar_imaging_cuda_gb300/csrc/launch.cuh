@@ -6,7 +6,10 @@
 // CTA of the kernel before has started and passed pdl_begin(), and wait there
 // until that kernel has completed and its writes are visible.  Whatever a
 // kernel does before pdl_begin() may touch shared memory and the context's
-// constant tables only.
+// constant tables only; the one exception is k_ra_spec0, which starts copying
+// the frame's echoes.  They are the caller's or an earlier kernel's, and the
+// kernel in front of it, k_zero_shift, is launched in the ordinary way: it
+// began only once all of that had completed, and does not touch them.
 //
 // Single frames use it; the lanes of a batch do not (a waiting CTA holds
 // shared memory and registers that another lane's kernel could use).  The

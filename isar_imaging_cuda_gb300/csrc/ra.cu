@@ -727,7 +727,9 @@ k_ra_spec0(const float2* x, float2* xw, const float* __restrict__ win, const int
         sb.issue(src + (size_t)(2 * j + 1) * kRowBytes, kRowBytes);
     }
     RaTw<N>::fill(twt, tw, lt, F::T);
-    pdl_begin();   // the echoes copied above are older than the kernel before
+    // The echoes copied above are older than the kernel before, k_zero_shift,
+    // which must stay an ordinary launch (launch.cuh).
+    pdl_begin();
     __syncthreads();
     const RaTw<N> tws{twt};
     const float invN = 1.0f / (float)N;
@@ -1379,6 +1381,8 @@ static cudaError_t ra_run_n(const RAArgs& a, cudaStream_t st)
     const int T = N / 16;
     int L = 0;
     while ((1 << L) < M) ++L;
+    // An ordinary launch: k_ra_spec0 behind it reads the echoes before its
+    // pdl_begin() (launch.cuh).
     k_zero_shift<<<(M + 255) / 256, 256, 0, st>>>(a.S, a.SQ, M, a.hmax);
     ISAR_COUNT(1);
     // spectral envelope merge: merged group spectra ping-pong between env_a
