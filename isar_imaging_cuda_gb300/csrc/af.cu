@@ -812,10 +812,11 @@ k_af_cluster(AFFrame f, int iters, float tol, const float2* __restrict__ tw)
     uint32_t par = 0;   // phase parity of both mbarriers: bit 0 bar_part, bit 1 bar_ph
     unsigned polls = f.polls;   // 0 once one of this thread's waits has run out
     auto await = [&](uint64_t* bar, uint32_t bit) {
-        if (msg_wait(bar, (par & bit) ? 1u : 0u, polls)) {
-            par ^= bit;
-        } else {
+        const uint32_t parity = (par & bit) ? 1u : 0u;
+        par ^= bit;
+        if (__builtin_expect(!msg_wait(bar, parity, polls), 0)) {
             polls = 0;
+            par ^= bit;
             atomicOr(f.err, 1u);
         }
     };
