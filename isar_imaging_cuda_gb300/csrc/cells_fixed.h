@@ -18,11 +18,14 @@ namespace isar {
 // ~16 clocks: with division, floor and scaling in double in every warp, and
 // three FP64 block sums, the range alignment of a 1024 x 8192 frame took
 // 33 us more (1556 -> 1523 us per frame; a batch of 32 learned frames 16.68 ->
-// 16.17 ms).
+// 16.17 ms).  A shift that is no number (the correlation with a missing pulse
+// has no peak to fit) or infinite is half a cycle, what the device's
+// double-to-integer conversion makes of it.
 ISAR_HD int64_t cells_to_fixed(uint64_t bits, int lgN)
 {
     const int ex = (int)((bits >> 52) & 0x7ff);
     if (ex == 0) return 0;                                     // zero (subnormals round to it)
+    if (ex == 0x7ff) return INT64_MIN;                         // NaN, infinity
     const uint64_t man = (bits & 0xfffffffffffffull) | 0x10000000000000ull;
     const int k = ex - 1075 + 64 - lgN;                        // v / N * 2^64 = man * 2^k
     uint64_t r;

@@ -65,3 +65,10 @@ def test_cells_to_fixed_is_exact(lib, lg):
     got = np.empty(v.size, np.int64)
     lib.convert(v.ctypes.data, got.ctypes.data, v.size, lg)
     assert got.tolist() == [exact_fixed(x, lg) for x in v.tolist()]
+
+
+def test_no_number_is_half_a_cycle(lib):
+    v = np.array([np.nan, -np.nan, np.inf, -np.inf])
+    got = np.empty(v.size, np.int64)
+    lib.convert(v.ctypes.data, got.ctypes.data, v.size, 13)
+    assert got.tolist() == [-(1 << 63)] * 4

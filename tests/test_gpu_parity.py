@@ -99,6 +99,28 @@ def test_range_align_stage(torch_cuda, gb300, M, N, hpc, rows_each_level):
     assert rel_l2(y2, y_want) < TOL_IMG
 
 
+# The pulse after a missing (zero) one in its pair gets no shift estimate; its
+# profile is the unaligned one, turned by half the range.
+@pytest.mark.parametrize("rows_each_level", [0, 1])
+def test_range_align_next_to_a_missing_pulse(torch_cuda, gb300, rows_each_level):
+    torch = torch_cuda
+    M, N, m = 128, 1024, 40
+    e, _ = make_frame(M, N, seed=17)
+    e = np.asarray(e, np.complex64).copy()
+    e[m] = 0
+    n = np.arange(N)
+    ham = 0.54 - 0.46 * np.cos(2.0 * np.pi * n / (N - 1))
+    want = np.roll(np.fft.ifft(e[m + 1].astype(np.complex128) * ham * np.cos(np.pi * n)), N // 2)
+    with ctx_for(gb300, torch, M, N) as ctx:
+        ctx.set_tuning(ra_rows_each_level=rows_each_level)
+        d = to_dev(torch, e)
+        ctx.stage_range_align(d)
+        y = from_dev(torch, d).reshape(M, N)
+        sh = ctx.trace()["ra_shift"]
+    assert np.isnan(sh[m // 2])
+    assert rel_l2(y[m + 1], want) < TOL_IMG
+
+
 # N = 512 and 8192 are the two ends of the centring sort (2 and 32 warps).
 @pytest.mark.parametrize("M,N", [(128, 512), (128, 1024), (256, 4096), (512, 8192)])
 def test_center_cut_stage(torch_cuda, gb300, M, N):
