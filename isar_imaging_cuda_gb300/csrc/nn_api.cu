@@ -126,6 +126,7 @@ ISAR_API int isar_wsnet_create(isar_wsnet** out, int max_rows, int training, int
     if (n->training) {
         for (int l = 0; l < kConv; ++l)
             if ((rc = nalloc(n.get(), &n->a.cols[l], R * kColK)) != ISAR_OK) return fin(rc);
+        n->a.act[0] = n->a.cols[0];   // a backward pass before any forward reads memory of the network
         if ((rc = nalloc(n.get(), &n->g.g, kParams)) != ISAR_OK) return fin(rc);
         if ((rc = nalloc(n.get(), &n->g.m1, kParams)) != ISAR_OK) return fin(rc);
         if ((rc = nalloc(n.get(), &n->g.m2, kParams)) != ISAR_OK) return fin(rc);

@@ -130,6 +130,23 @@ def test_grads_match_oracle_at_row_block_edges(torch_cuda, gb300, F, M):
             assert np.linalg.norm(a - w) / max(np.linalg.norm(w), 1e-30) < 1e-3, (li, name)
 
 
+# Before any forward there is nothing to differentiate, but the call is accepted
+# and what follows is not affected.
+@pytest.mark.parametrize("F,M", [(2, 128), (2, 72)])
+def test_backward_before_any_forward(torch_cuda, gb300, F, M):
+    torch = torch_cuda
+    p, _, _, dx, dt = _setup(torch, F, M, 9)
+    out = []
+    for early in (True, False):
+        with gb300.WSNet(F * M, training=True) as net:
+            net.set_params(p)
+            if early:
+                net.backward(dt, F, M)
+            net.forward(dx, F, M)
+            out.append(net.backward(dt, F, M))
+    assert out[0] == out[1]
+
+
 def test_adam_steps_reduce_loss(torch_cuda, gb300):
     torch = torch_cuda
     F, M = 8, 64
